@@ -40,7 +40,7 @@ namespace fbc {
 constexpr int32_t kInf = 0x7fffffff;
 constexpr unsigned kFull = 0xffffffffu;
 
-enum : int { kErrIter = 1, kErrSigma = 2, kErrQueue = 4, kErrRetry = 8 };
+enum : int { kErrIter = 1, kErrSigma = 2, kErrQueue = 4, kErrRetry = 8, kErrNarrow = 16 };
 
 // One CSR segment (device pointers).
 struct Seg {
@@ -68,7 +68,8 @@ struct Unit {
 
 // A unit whose path counts outgrew the kernel's representation.  It stopped before its
 // dependency pass (nothing accumulated) and the host recomputes it one level up:
-// code kErrRetry -> plain kernel with 64-bit counts, kErrSigma -> plain kernel with FP64
+// code kErrNarrow (team kernel) -> shared-memory or frontier kernel, kErrRetry -> plain kernel with
+// 64-bit counts, kErrSigma -> plain kernel with FP64
 // counts (the reference's own representation, exact below 2^53).
 struct RetryRec {
     Unit u;
@@ -104,7 +105,7 @@ struct KParams {
 // Hand a unit back to the host (see RetryRec); without a retry list, report the error.
 __device__ __forceinline__ void request_retry(const KParams& P, const Unit& u, int code) {
     if (!P.retry) {
-        atomicOr(P.err, code == kErrRetry ? kErrSigma : code);
+        atomicOr(P.err, kErrSigma);
         return;
     }
     const int r = atomicAdd(P.retry_count, 1);
@@ -184,6 +185,17 @@ struct PrecF64 {
     __device__ static Acc load(D d) { return {d}; }
     __device__ static double value(const Acc& a) { return a.s; }
     __device__ static void red_add(double* p, const Acc& a) { atomicAdd(p, a.s); }
+    // The team kernel's form: coefficient (1 + delta) / sigma of a vertex, their sum over the tight
+    // out-edges, and sigma times that sum.  Division by a power of two is an exact scaling.
+    __device__ static D coef1(const Acc& d) { return 1.0 + d.s; }  // sigma 1
+    __device__ static D coef(const Acc& d, unsigned long long s) {
+        const double t = 1.0 + d.s;
+        if (s == 1ull) return t;
+        if ((s & (s - 1ull)) == 0ull) return t * __longlong_as_double((long long)(1023 - (63 - __clzll((long long)s))) << 52);
+        return t / (double)s;
+    }
+    __device__ static void add_coefs(Acc& a, D c0, D c1, D c2, D c3) { a.s = a.s + c0 + c1 + c2 + c3; }
+    __device__ static Acc times(const Acc& a, unsigned long long s) { return s == 1ull ? a : Acc{a.s * (double)s}; }
 };
 
 struct PrecDF32 {
@@ -260,6 +272,60 @@ struct PrecDF32 {
     __device__ static D store(const Acc& a) { return make_float2(a.hi, a.lo); }
     __device__ static Acc load(D d) { return {d.x, d.y}; }
     __device__ static double value(const Acc& a) { return (double)a.hi + (double)a.lo; }
+    // the team kernel's form (see PrecF64::coef)
+    __device__ static D coef1(const Acc& d) {
+        float sum, e, th, tl;
+        two_sum(1.0f, d.hi, sum, e);
+        e = __fadd_rn(e, d.lo);
+        fast_two_sum(sum, e, th, tl);
+        return make_float2(th, tl);
+    }
+    __device__ static D coef(const Acc& d, unsigned long long s) {
+        float sum, e, th, tl;
+        two_sum(1.0f, d.hi, sum, e);
+        e = __fadd_rn(e, d.lo);
+        fast_two_sum(sum, e, th, tl);
+        if (s == 1ull) return make_float2(th, tl);
+        if ((s & (s - 1ull)) == 0ull) {
+            const float f = __int_as_float((127 - (63 - __clzll((long long)s))) << 23);
+            return make_float2(__fmul_rn(th, f), __fmul_rn(tl, f));
+        }
+        float ch, cl;
+        if (s <= 16777216ull) {
+            const float y = __uint2float_rn((unsigned)s);
+            ch = __fdiv_rn(th, y);
+            cl = __fdiv_rn(__fadd_rn(__fmaf_rn(-ch, y, th), tl), y);  // th - ch*y is exact
+            fast_two_sum(ch, cl, th, tl);
+            return make_float2(th, tl);
+        }
+        const double q = ((double)th + (double)tl) / (double)s;
+        ch = __double2float_rn(q);
+        return make_float2(ch, __double2float_rn(q - (double)ch));
+    }
+    __device__ static void add_coefs(Acc& a, D c0, D c1, D c2, D c3) {
+        float e, f, g, h;
+        two_sum(a.hi, c0.x, a.hi, e);
+        two_sum(a.hi, c1.x, a.hi, f);
+        two_sum(a.hi, c2.x, a.hi, g);
+        two_sum(a.hi, c3.x, a.hi, h);
+        const float lo = __fadd_rn(__fadd_rn(__fadd_rn(c0.y, e), __fadd_rn(c1.y, f)),
+                                   __fadd_rn(__fadd_rn(c2.y, g), __fadd_rn(c3.y, h)));
+        fast_two_sum(a.hi, __fadd_rn(a.lo, lo), e, f);
+        a = {e, f};
+    }
+    __device__ static Acc times(const Acc& a, unsigned long long s) {
+        if (s == 1ull) return a;
+        if (s <= 16777216ull) {
+            const float y = __uint2float_rn((unsigned)s);
+            const float p = __fmul_rn(a.hi, y);
+            Acc r;
+            fast_two_sum(p, __fadd_rn(__fmaf_rn(a.hi, y, -p), __fmul_rn(a.lo, y)), r.hi, r.lo);
+            return r;
+        }
+        const double q = ((double)a.hi + (double)a.lo) * (double)s;
+        const float h = __double2float_rn(q);
+        return {h, __double2float_rn(q - (double)h)};
+    }
     // BC[o] += value: the halves widened by integer ops (the same doubles as a conversion) and
     // reduced one after the other, so the cross-source sum is the only FP64 arithmetic, done by
     // the reductions in L2 (the FP64 pipe stays idle)

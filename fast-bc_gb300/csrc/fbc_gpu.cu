@@ -28,6 +28,7 @@
 #include "text_parse.cuh"
 #include "frontier_kernels.cuh"
 #include "kmeans.cuh"
+#include "team_kernels.cuh"
 #include "host_order.hpp"
 
 namespace {
@@ -133,6 +134,8 @@ struct Ctx {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, evm = nullptr;
     Options opt;
     DBuf retry, segs, units_b, units_w, chunks, crp, cadj, cgid, cbord, bc, bdist, bsig, ctr, dbg, bcseg;
+    // team kernel: segment list, quads, continuation counts, units and work items of its launches
+    DBuf tsegs, tquad, textra, tunits, tchunks;
     // cluster extraction scratch: offsets, ids, flags, scans, given borders, error word
     DBuf c_off, c_id, c_lid, c_isb, c_flag, c_scan, c_sums, c_boff, c_bsrc, c_m, c_err;
     Workspace wsb, wsw;
@@ -167,6 +170,7 @@ struct fbc_graph_s {
     int64_t m = 0;
     int32_t maxw = 0;
     int32_t maxindeg = 0;
+    int32_t maxdeg = 0;  // longest row
     double meanw = 1.0;
     int32_t* d_rp = nullptr;
     int2* d_adj = nullptr;
@@ -193,6 +197,9 @@ struct fbc_plan_s {
     int prec = FBC_PREC_FP32C;
     int64_t n = 0, ent = 0;
     DBuf crp, cadj, cgid, cbord, segs, units, chunks, bc, bdist, bsig, ctr, retry, bunits, ws;
+    struct Team {  // one team launch: communities up to warp_max_n, and above it
+        DBuf segs, quad, extra, units, chunks;
+    } team[2];
     double* h_bc = nullptr;
     double* h_bdist = nullptr;
     uint64_t* h_bsig = nullptr;
@@ -219,6 +226,8 @@ struct fbc_plan_s {
         for (DBuf* b : {&crp, &cadj, &cgid, &cbord, &segs, &units, &chunks, &bc, &bdist, &bsig, &ctr, &retry,
                         &bunits, &ws})
             b->release();
+        for (Team& t : team)
+            for (DBuf* b : {&t.segs, &t.quad, &t.extra, &t.units, &t.chunks}) b->release();
         if (h_bc) cudaFreeHost(h_bc);
         if (h_bdist) cudaFreeHost(h_bdist);
         if (h_bsig) cudaFreeHost(h_bsig);
@@ -244,9 +253,11 @@ int make_graph(int32_t n, std::vector<int64_t>&& rp, std::vector<int32_t>&& col,
     if (m < 0 || m >= (int64_t)0x7fffffff) return fail(FBC_ERR_RANGE, "edge count outside [0, 2^31-1)");
     std::vector<int32_t> wi((size_t)m);
     int32_t maxw = 0;
+    int64_t maxdeg = 0;
     double sumw = 0;
     for (int32_t v = 0; v < n; ++v) {
         if (rp[v + 1] < rp[v]) return fail(FBC_ERR_INVALID_ARG, "row_ptr is not monotone");
+        maxdeg = std::max(maxdeg, rp[v + 1] - rp[v]);
         for (int64_t e = rp[v]; e < rp[v + 1]; ++e) {
             if (col[e] < 0 || col[e] >= n)
                 return fail(FBC_ERR_INVALID_ARG,
@@ -269,6 +280,7 @@ int make_graph(int32_t n, std::vector<int64_t>&& rp, std::vector<int32_t>&& col,
     for (int64_t e = 0; e < m; ++e) indeg[col[e]]++;
     auto* G = new fbc_graph_s();
     G->maxindeg = n ? *std::max_element(indeg.begin(), indeg.begin() + n) : 0;
+    G->maxdeg = (int32_t)maxdeg;
     G->n = n;
     G->m = m;
     G->maxw = maxw;
@@ -314,6 +326,7 @@ struct Plan {
     std::vector<int64_t> seg_m;
     std::vector<int32_t> seg_maxw;
     std::vector<int32_t> seg_maxindeg;
+    std::vector<int32_t> seg_maxdeg;
     std::vector<Unit> units;
     int64_t bc_len = 0;
     int64_t border_entries = 0;
@@ -728,11 +741,222 @@ int launch_small(const Plan& P, const std::vector<Unit>& units, int nmax, int mm
     return FBC_OK;
 }
 
+// ---- team kernel (team_kernels.cuh): segments whose per-source state fits shared memory ----
+int64_t team_dyn_smem() { return (int64_t)g.smem_optin - 1024; }  // its control words are static
+
+int bit_length(uint64_t x) {
+    int b = 0;
+    while (x) { ++b; x >>= 1; }
+    return b;
+}
+
+// What the kernel's packed forms hold: 16-bit byte offsets of vertices, 16-bit quad numbers, 15-bit
+// weights, rows of up to 16 edges, 255 in-edges at most (sums of counts below 2^24), distances that
+// leave a word eight stamp bits; and two sources' state in a block's shared memory (with one, the
+// frontier kernel is faster: 47 against 55 ms for the sources of a 16,384-vertex grid).
+// Graphs of tiny weights (kTeamMinMaxW) have many tied paths, whose counts outgrow the kernel's
+// on most sources: they stay with the kernels of wider counts.
+constexpr int64_t kTeamMinMaxW = 8;
+bool team_fits(const Plan& P, size_t s) {
+    const int64_t n = P.segs[s].n, maxw = P.seg_maxw[s];
+    return n >= 1 && n <= fbc::kTeamMaxN && P.seg_maxdeg[s] <= fbc::kTeamRow && P.seg_maxindeg[s] <= fbc::kTeamIndeg &&
+           maxw >= kTeamMinMaxW && maxw < 32768 && bit_length((uint64_t)n * (uint64_t)maxw + 1) <= fbc::kTeamDistBits &&
+           n + P.seg_m[s] / 3 + 1 <= 65535 && 2 * fbc::team_bytes(n, P.seg_maxdeg[s] > 8) <= team_dyn_smem();
+}
+
+// Segments above warp_max_n go to the team kernel too, unless an option asks for the frontier
+// kernel: warp_max_n = 0 (no segment in shared memory) or a forced number of sources per block.
+bool team_takes_blocks() { return g.opt.warp_max_n > 0 && g.opt.group == 0; }
+
+// Host side of a team launch: the segments with their quads, and the (segment, sources) items,
+// largest segments first.
+struct TeamCfg {
+    std::vector<fbc::TeamSeg> segs;
+    std::vector<int64_t> quad_off;  // first quad of each
+    int64_t nquads = 0;
+    int nmax = 0;
+    std::vector<Unit> units;        // grouped by segment
+    std::vector<fbc::Chunk> chunks;
+    int64_t blocks = 0;
+};
+
+// `units` grouped by segment.
+void team_config(const Plan& P, std::vector<Unit>&& units, TeamCfg& c) {
+    c = TeamCfg{};
+    c.units = std::move(units);
+    double work = 0;
+    for (const Unit& u : c.units) work += P.segs[u.seg].n;
+    const double per_sm = work / std::max(1, g.nsm);
+    for (size_t i = 0; i < c.units.size();) {
+        const int32_t seg = c.units[i].seg;
+        size_t j = i;
+        while (j < c.units.size() && c.units[j].seg == seg) ++j;
+        const int64_t n = P.segs[seg].n;
+        fbc::TeamSeg t{};
+        t.seg = seg;
+        t.stamp_bits = 32 - bit_length((uint64_t)n * (uint64_t)P.seg_maxw[seg] + 1);
+        t.stamp_bits = std::min(t.stamp_bits, 24);
+        t.wide_mask = P.seg_maxdeg[seg] > 8;
+        c.quad_off.push_back(c.nquads);
+        c.nquads += n + P.seg_m[seg] / 3 + 1;
+        c.nmax = std::max<int>(c.nmax, (int)n);
+        const int32_t ti = (int32_t)c.segs.size();
+        c.segs.push_back(t);
+        // sources per item: about eight items for every SM, each a few times what a block runs at
+        // once (the block waits for its last source before it takes the next item), but never so
+        // many that an SM is left without one
+        const int64_t at_once = std::max<int64_t>(1, team_dyn_smem() / (fbc::team_bytes(n, t.wide_mask) + 16));
+        const int64_t fair = std::max<int64_t>(1, (int64_t)std::ceil(per_sm / (double)n));
+        int64_t per = std::max<int64_t>((int64_t)(per_sm / (8.0 * (double)n)), std::min<int64_t>(4 * at_once, fair));
+        per = std::max<int64_t>(1, std::min<int64_t>(per, g.opt.chunk_max));
+        for (size_t k = i; k < j; k += (size_t)per)
+            c.chunks.push_back(fbc::Chunk{ti, (int32_t)k, (int32_t)std::min<int64_t>(per, (int64_t)(j - k)), 0});
+        i = j;
+    }
+    std::stable_sort(c.chunks.begin(), c.chunks.end(), [&](const fbc::Chunk& a, const fbc::Chunk& b) {
+        return P.segs[c.segs[a.seg].seg].n > P.segs[c.segs[b.seg].seg].n;
+    });
+    c.blocks = std::min<int64_t>((int64_t)g.nsm, (int64_t)c.chunks.size());
+}
+
+// Upload a team launch's lists into the given buffers and build its quads from the segments'
+// CSRs (dsegs: the uploaded segment list).
+int team_upload(TeamCfg& c, const Seg* dsegs, DBuf& tsegs, DBuf& tquad, DBuf& textra, DBuf& tunits, DBuf& tchunks,
+                fbc_stats* st) {
+    FBC_CK(tsegs.ensure(sizeof(fbc::TeamSeg) * c.segs.size()));
+    FBC_CK(tquad.ensure(sizeof(uint4) * (size_t)c.nquads));
+    FBC_CK(textra.ensure(sizeof(int32_t) * c.segs.size()));
+    FBC_CK(tunits.ensure(sizeof(Unit) * c.units.size()));
+    FBC_CK(tchunks.ensure(sizeof(fbc::Chunk) * c.chunks.size()));
+    for (size_t i = 0; i < c.segs.size(); ++i) c.segs[i].quad = tquad.as<uint4>() + c.quad_off[i];
+    FBC_CK(cudaMemcpyAsync(tsegs.p, c.segs.data(), sizeof(fbc::TeamSeg) * c.segs.size(), cudaMemcpyHostToDevice, g.st));
+    FBC_CK(cudaMemcpyAsync(tunits.p, c.units.data(), sizeof(Unit) * c.units.size(), cudaMemcpyHostToDevice, g.st));
+    FBC_CK(cudaMemcpyAsync(tchunks.p, c.chunks.data(), sizeof(fbc::Chunk) * c.chunks.size(), cudaMemcpyHostToDevice, g.st));
+    FBC_CK(cudaMemsetAsync(textra.p, 0, sizeof(int32_t) * c.segs.size(), g.st));
+    const dim3 grid((unsigned)c.segs.size(), (unsigned)std::max(1, std::min(64, (c.nmax + 255) / 256)));
+    fbc::team_quads_kernel<<<grid, 256, 0, g.st>>>(dsegs, tsegs.as<fbc::TeamSeg>(), textra.as<int32_t>());
+    FBC_CK(cudaGetLastError());
+    if (st)
+        st->h2d_bytes += (int64_t)(sizeof(fbc::TeamSeg) * c.segs.size() + sizeof(Unit) * c.units.size() +
+                                   sizeof(fbc::Chunk) * c.chunks.size());
+    return FBC_OK;
+}
+
+fbc::TeamParams team_params(const TeamCfg& c, const KParams& base, DBuf& tsegs, DBuf& textra, DBuf& tunits,
+                            DBuf& tchunks, unsigned long long* next_chunk) {
+    fbc::TeamParams T{};
+    T.k = base;
+    T.k.units = tunits.as<Unit>();
+    T.k.nunits = (int64_t)c.units.size();
+    T.tsegs = tsegs.as<fbc::TeamSeg>();
+    T.extra = textra.as<int32_t>();
+    T.chunks = tchunks.as<fbc::Chunk>();
+    T.nchunks = (int32_t)c.chunks.size();
+    T.smem = (int32_t)team_dyn_smem();
+    T.next_chunk = next_chunk;
+    return T;
+}
+
+template <class Prec>
+int team_launch(const TeamCfg& c, const fbc::TeamParams& T) {
+    auto kern = fbc::team_kernel<Prec>;
+    FBC_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T.smem));
+    kern<<<(unsigned)c.blocks, fbc::kTeamThreads, (size_t)T.smem, g.st>>>(T);
+    FBC_CK(cudaGetLastError());
+    return FBC_OK;
+}
+
+// A team launch on the library's buffers.
+template <class Prec>
+int launch_team(const Plan& P, std::vector<Unit>&& units, fbc_stats* st, int& launches) {
+    if (units.empty()) return FBC_OK;
+    TeamCfg c;
+    team_config(P, std::move(units), c);
+    FBC_TRY(team_upload(c, g.segs.as<Seg>(), g.tsegs, g.tquad, g.textra, g.tunits, g.tchunks, st));
+    FBC_TRY(team_launch<Prec>(c, team_params(c, base_params(P), g.tsegs, g.textra, g.tunits, g.tchunks,
+                                             g.ctr.as<unsigned long long>() + 1)));
+    launches += 2;
+    return FBC_OK;
+}
+
 int map_err(int e) {
     if (e & fbc::kErrQueue) return fail(FBC_ERR_QUEUE, "device work queue overflow");
     if (e & fbc::kErrIter) return fail(FBC_ERR_ITER_LIMIT, "a device loop reached its iteration bound");
     if (e & fbc::kErrSigma) return fail(FBC_ERR_SIGMA_OVERFLOW, "a shortest-path count exceeded 2^64-1");
     return FBC_OK;
+}
+
+// Units of the kernels besides the team kernel: one warp per source in shared memory (grouped by
+// segment), or block-per-source (biggest segments first).
+struct OldSplit {
+    std::vector<Unit> uw, ub;
+    int nb_max = 0, nw_max = 0, mw_max = 0, nw_min = 1 << 30;
+};
+
+void split_old(Plan& P, const std::vector<Unit>& units, OldSplit& o) {
+    std::vector<char> small(P.segs.size(), 0);
+    if (P.sched == FBC_SCHED_BATCHED && !P.dbg_dist)
+        for (const Unit& u : units) {
+            const size_t s = (size_t)u.seg;
+            small[s] = P.segs[s].n <= std::min<int64_t>(g.opt.warp_max_n, 65535) && P.seg_maxw[s] < 65536 &&
+                       P.seg_m[s] < ((int64_t)1 << 30);
+        }
+    // the shared-memory layout is sized by the largest small segment: demote the largest
+    // ones until at least two warps fit
+    for (;;) {
+        int nm = 0, mm = 0, arg = -1;
+        for (size_t s = 0; s < P.segs.size(); ++s)
+            if (small[s]) {
+                mm = std::max<int>(mm, (int)P.seg_m[s]);
+                if (P.segs[s].n >= nm) { nm = P.segs[s].n; arg = (int)s; }
+            }
+        if (arg < 0 || small_fits(nm, mm, 2)) break;
+        small[arg] = 0;
+    }
+    std::vector<std::vector<Unit>> by_seg(P.segs.size());
+    for (const Unit& u : units) {
+        if (small[u.seg]) {
+            by_seg[u.seg].push_back(u);
+            o.nw_max = std::max(o.nw_max, P.segs[u.seg].n);
+            o.nw_min = std::min(o.nw_min, P.segs[u.seg].n);
+            o.mw_max = std::max<int>(o.mw_max, (int)P.seg_m[u.seg]);
+        } else {
+            o.ub.push_back(u);
+            o.nb_max = std::max(o.nb_max, P.segs[u.seg].n);
+        }
+    }
+    for (auto& v : by_seg) o.uw.insert(o.uw.end(), v.begin(), v.end());
+    std::stable_sort(o.ub.begin(), o.ub.end(), [&](const Unit& a, const Unit& b) {
+        return P.segs[a.seg].n > P.segs[b.seg].n;
+    });
+    // the batched block kernel keeps tight in-edge counts in at most 16 bits
+    if (P.sched == FBC_SCHED_BATCHED)
+        for (const Unit& u : o.ub)
+            if (P.seg_maxindeg[u.seg] >= 65535) {
+                P.sched = FBC_SCHED_PLAIN;
+                break;
+            }
+}
+
+// The block-per-source launches.  Batched: segments of up to 32K vertices run in a launch of their
+// own (where several sources share a block, their rounds and levels), the larger ones one source
+// per block.
+template <class Prec>
+int launch_old_blocks(const Plan& P, const OldSplit& o, fbc_stats* st, int& launches) {
+    std::vector<Unit> us_small, us_large;
+    int ns_max = 0, nl_max = 0;
+    if (P.sched == FBC_SCHED_BATCHED && !P.dbg_dist)
+        for (const Unit& u : o.ub) {
+            const int sn = P.segs[u.seg].n;
+            if (sn <= 32768) { us_small.push_back(u); ns_max = std::max(ns_max, sn); }
+            else { us_large.push_back(u); nl_max = std::max(nl_max, sn); }
+        }
+    if (us_small.empty() || us_large.empty()) return launch_block<Prec>(P, o.ub, o.nb_max, st, launches);
+    // the launch with the larger slot layout first, so that the second reuses it
+    const bool small_first = (int64_t)ns_max * 4 >= (int64_t)nl_max;
+    FBC_TRY(launch_block<Prec>(P, small_first ? us_small : us_large, small_first ? ns_max : nl_max, st, launches));
+    FBC_CK(cudaMemsetAsync(g.ctr.p, 0, 8, g.st));  // the unit counter of the next launch
+    return launch_block<Prec>(P, small_first ? us_large : us_small, small_first ? nl_max : ns_max, st, launches);
 }
 
 // Upload the plan, launch, wait, and check the device status.  Results stay on the device
@@ -747,101 +971,79 @@ int run_plan_t(Plan& P, fbc_stats* st) {
     FBC_CK(cudaMemsetAsync(g.ctr.p, 0, 64, g.st));
     if (st) st->h2d_bytes += (int64_t)(sizeof(Seg) * P.segs.size());
 
-    // split units by schedule.  Batched: segments that fit the shared-memory kernel run
-    // there (grouped by segment); the rest run block-per-source, biggest segments first.
-    std::vector<Unit> ub, uw;
-    int nb_max = 0, nw_max = 0, mw_max = 0;
-    std::vector<char> small(P.segs.size(), 0);
+    // split units by kernel.  Batched: segments that fit the team kernel run there, up to
+    // warp_max_n in one launch (with what the one-warp kernel takes, the first timed phase) and
+    // above it in another; the rest run block-per-source.
+    std::vector<Unit> rest, tw, tb;
+    std::vector<char> team(P.segs.size(), 0);
     if (P.sched == FBC_SCHED_BATCHED && !P.dbg_dist) {  // debug dumps come from block kernels
-        for (size_t s = 0; s < P.segs.size(); ++s) {
-            const int n = P.segs[s].n;
-            small[s] = n <= std::min<int64_t>(g.opt.warp_max_n, 65535) && P.seg_maxw[s] < 65536 &&
-                       P.seg_m[s] < ((int64_t)1 << 30);
-        }
-    }
-    // the shared-memory layout is sized by the largest small segment: demote the largest
-    // ones until at least two warps fit
-    for (;;) {
-        int nm = 0, mm = 0, arg = -1;
+        const bool blocks = team_takes_blocks();
         for (size_t s = 0; s < P.segs.size(); ++s)
-            if (small[s]) {
-                mm = std::max<int>(mm, (int)P.seg_m[s]);
-                if (P.segs[s].n >= nm) { nm = P.segs[s].n; arg = (int)s; }
-            }
-        if (arg < 0 || small_fits(nm, mm, 2)) break;
-        small[arg] = 0;
+            team[s] = (P.segs[s].n <= std::min<int64_t>(g.opt.warp_max_n, 65535) || blocks) && team_fits(P, s);
     }
-    int nw_min = 1 << 30;
-    std::vector<std::vector<Unit>> by_seg(P.segs.size());
+    int64_t nwarp = 0, nblock = 0;  // units of the two phases
+    double warp_bytes = 0, block_bytes = 0;
     for (const Unit& u : P.units) {
-        if (small[u.seg]) {
-            by_seg[u.seg].push_back(u);
-            nw_max = std::max(nw_max, P.segs[u.seg].n);
-            nw_min = std::min(nw_min, P.segs[u.seg].n);
-            mw_max = std::max<int>(mw_max, (int)P.seg_m[u.seg]);
-        } else {
-            ub.push_back(u);
-            nb_max = std::max(nb_max, P.segs[u.seg].n);
+        if (!team[u.seg]) {
+            rest.push_back(u);
+            continue;
         }
+        const bool up_to = P.segs[u.seg].n <= g.opt.warp_max_n;
+        (up_to ? tw : tb).push_back(u);
+        (up_to ? nwarp : nblock) += 1;
+        (up_to ? warp_bytes : block_bytes) += 40.0 * (double)P.seg_m[u.seg] + 52.0 * P.segs[u.seg].n;
     }
-    for (auto& v : by_seg) uw.insert(uw.end(), v.begin(), v.end());
-    std::stable_sort(ub.begin(), ub.end(), [&](const Unit& a, const Unit& b) {
-        return P.segs[a.seg].n > P.segs[b.seg].n;
-    });
-    // the batched block kernel keeps tight in-edge counts in at most 16 bits
-    if (P.sched == FBC_SCHED_BATCHED)
-        for (const Unit& u : ub)
-            if (P.seg_maxindeg[u.seg] >= 65535) {
-                P.sched = FBC_SCHED_PLAIN;
-                break;
-            }
+    for (std::vector<Unit>* v : {&tw, &tb})
+        std::stable_sort(v->begin(), v->end(), [](const Unit& a, const Unit& b) { return a.seg < b.seg; });
+    OldSplit sp;
+    split_old(P, rest, sp);
+    nwarp += (int64_t)sp.uw.size();
+    nblock += (int64_t)sp.ub.size();
+    for (const Unit& u : sp.uw) warp_bytes += 40.0 * (double)P.seg_m[u.seg] + 52.0 * P.segs[u.seg].n;
+    for (const Unit& u : sp.ub) block_bytes += 40.0 * (double)P.seg_m[u.seg] + 52.0 * P.segs[u.seg].n;
     FBC_CK(g.segs.ensure(sizeof(Seg) * std::max<size_t>(P.segs.size(), 1)));
     FBC_CK(cudaMemcpyAsync(g.segs.p, P.segs.data(), sizeof(Seg) * P.segs.size(),
                            cudaMemcpyHostToDevice, g.st));
     int launches = 0;
     FBC_CK(cudaEventRecord(g.ev0, g.st));
     FBC_CK(g.retry.ensure(sizeof(fbc::RetryRec) * std::max<size_t>(P.units.size(), 1)));
-    FBC_TRY(launch_small<Prec>(P, uw, nw_max, mw_max, nw_min, st, launches));
+    FBC_TRY(launch_small<Prec>(P, sp.uw, sp.nw_max, sp.mw_max, sp.nw_min, st, launches));
+    if (!sp.uw.empty() && !tw.empty()) FBC_CK(cudaMemsetAsync(g.ctr.as<unsigned long long>() + 1, 0, 8, g.st));
+    FBC_TRY(launch_team<Prec>(P, std::move(tw), st, launches));
     FBC_CK(cudaEventRecord(g.evm, g.st));
-    {
-        // batched: segments of up to 32K vertices run in a launch of their own (where several
-        // sources share a block, their rounds and levels), the larger ones one source per block
-        std::vector<Unit> us_small, us_large;
-        int ns_max = 0, nl_max = 0;
-        if (P.sched == FBC_SCHED_BATCHED && !P.dbg_dist)
-            for (const Unit& u : ub) {
-                const int sn = P.segs[u.seg].n;
-                if (sn <= 32768) { us_small.push_back(u); ns_max = std::max(ns_max, sn); }
-                else { us_large.push_back(u); nl_max = std::max(nl_max, sn); }
-            }
-        if (!us_small.empty() && !us_large.empty()) {
-            // the launch with the larger slot layout first, so that the second reuses it
-            const bool small_first = (int64_t)ns_max * 4 >= (int64_t)nl_max;
-            FBC_TRY(launch_block<Prec>(P, small_first ? us_small : us_large, small_first ? ns_max : nl_max, st, launches));
-            FBC_CK(cudaMemsetAsync(g.ctr.p, 0, 8, g.st));  // the unit counter of the next launch
-            FBC_TRY(launch_block<Prec>(P, small_first ? us_large : us_small, small_first ? nl_max : ns_max, st, launches));
-        } else {
-            FBC_TRY(launch_block<Prec>(P, ub, nb_max, st, launches));
-        }
+    if (!tb.empty()) {
+        FBC_CK(cudaMemsetAsync(g.ctr.as<unsigned long long>() + 1, 0, 8, g.st));
+        FBC_TRY(launch_team<Prec>(P, std::move(tb), st, launches));
     }
+    FBC_TRY(launch_old_blocks<Prec>(P, sp, st, launches));
     int err[2] = {0, 0};
     FBC_CK(cudaMemcpyAsync(err, (char*)g.ctr.p + 16, 2 * sizeof(int), cudaMemcpyDeviceToHost, g.st));
     FBC_CK(cudaStreamSynchronize(g.st));
     // Units whose path counts outgrew their kernel's representation stopped before their
     // dependency pass (nothing of theirs was accumulated): recompute them one level up,
-    // 48-bit packed -> 64-bit (plain kernel) -> FP64 counts (plain kernel).
-    for (int round = 0; round < 3 && err[0] == 0 && err[1] > 0; ++round) {
+    // 32-bit (team kernel) -> shared-memory or frontier kernel, packed -> 64-bit (plain kernel) -> FP64
+    // counts (plain kernel).
+    for (int round = 0; round < 4 && err[0] == 0 && err[1] > 0; ++round) {
         std::vector<fbc::RetryRec> rec((size_t)err[1]);
         if (st) st->retries += err[1];
         FBC_CK(cudaMemcpy(rec.data(), g.retry.p, sizeof(fbc::RetryRec) * rec.size(), cudaMemcpyDeviceToHost));
-        std::vector<Unit> to64, tof64;
+        std::vector<Unit> to64, tof64, narrow;
         int nmax = 0;
         for (const auto& r : rec) {
-            (r.code == fbc::kErrRetry ? to64 : tof64).push_back(r.u);
+            (r.code == fbc::kErrNarrow ? narrow : r.code == fbc::kErrRetry ? to64 : tof64).push_back(r.u);
             nmax = std::max(nmax, P.segs[r.u.seg].n);
         }
+        if (!narrow.empty()) {  // counts above the team kernel's 32 bits: the kernels with wider ones
+            OldSplit ns;
+            split_old(P, narrow, ns);
+            FBC_CK(cudaMemsetAsync(g.ctr.p, 0, 16, g.st));
+            FBC_CK(cudaMemsetAsync((char*)g.ctr.p + 20, 0, 4, g.st));
+            FBC_TRY(launch_small<Prec>(P, ns.uw, ns.nw_max, ns.mw_max, ns.nw_min, st, launches));
+            FBC_TRY(launch_old_blocks<Prec>(P, ns, st, launches));
+        } else {
+            FBC_CK(cudaMemsetAsync((char*)g.ctr.p + 20, 0, 4, g.st));
+        }
         FBC_CK(cudaMemsetAsync(g.ctr.p, 0, 8, g.st));
-        FBC_CK(cudaMemsetAsync((char*)g.ctr.p + 20, 0, 4, g.st));
         FBC_TRY(launch_block<Prec>(P, to64, nmax, st, launches, true, false));
         if (!to64.empty() && !tof64.empty()) {
             FBC_CK(cudaMemsetAsync(g.ctr.p, 0, 8, g.st));
@@ -860,12 +1062,12 @@ int run_plan_t(Plan& P, fbc_stats* st) {
         FBC_CK(cudaEventElapsedTime(&mw, g.ev0, g.evm));
         FBC_CK(cudaEventElapsedTime(&mb, g.evm, g.ev1));
         st->kernel_ms += ms;
-        st->warp_ms += uw.empty() ? 0.0 : mw;
-        st->block_ms += ub.empty() ? 0.0 : mb;
-        st->warp_units += (int64_t)uw.size();
-        st->block_units += (int64_t)ub.size();
-        for (const Unit& u : uw) st->warp_bytes += 40.0 * (double)P.seg_m[u.seg] + 52.0 * P.segs[u.seg].n;
-        for (const Unit& u : ub) st->block_bytes += 40.0 * (double)P.seg_m[u.seg] + 52.0 * P.segs[u.seg].n;
+        st->warp_ms += nwarp ? mw : 0.0;
+        st->block_ms += nblock ? mb : 0.0;
+        st->warp_units += nwarp;
+        st->block_units += nblock;
+        st->warp_bytes += warp_bytes;
+        st->block_bytes += block_bytes;
         st->units += (int64_t)P.units.size();
         double rel = 0;
         for (const Unit& u : P.units) rel += (double)P.seg_m[u.seg];
@@ -1122,6 +1324,7 @@ int prepare_clusters(const fbc_graph_s* G, int32_t nclusters, const int64_t* cof
         P.seg_m.push_back(seg_m[c]);
         P.seg_maxw.push_back(G->maxw);
         P.seg_maxindeg.push_back(G->maxindeg);
+        P.seg_maxdeg.push_back(G->maxdeg);
         for (int32_t i = 0; i < s.n; ++i) P.units.push_back(Unit{c, i, 1.0, ent + (int64_t)i * s.nb});
         ent += (int64_t)s.n * s.nb;
     }
@@ -1172,8 +1375,9 @@ int device_csr_build(int64_t count, const int32_t* dsrc, const int32_t* ddst, co
     *out = nullptr;
     TmpBuf ints, deg, rs, cursor, keys, ndeg, indeg;
     FBC_CK(ints.ensure(64));
-    // ints: [0] max source, [1] error bits, [2] max weight, [3] max in-degree, [4..5] weight sum
-    int hi[6] = {-1, 0, 0, 0, 0, 0};
+    // ints: [0] max source, [1] error bits, [2] max weight, [3] max in-degree, [4..5] weight sum,
+    // [6] longest row
+    int hi[7] = {-1, 0, 0, 0, 0, 0, 0};
     FBC_CK(cudaMemcpyAsync(ints.p, hi, sizeof(hi), cudaMemcpyHostToDevice, g.st));
     int* di = ints.as<int>();
     fbc::gb_check_kernel<<<grid_for(count), 256, 0, g.st>>>(count, dsrc, ddst,
@@ -1235,7 +1439,7 @@ int device_csr_build(int64_t count, const int32_t* dsrc, const int32_t* ddst, co
     }
     fbc::gb_merge_kernel<<<grid_for(n), 256, 0, g.st>>>(n, rs.as<int32_t>(), keys.as<unsigned long long>(),
                                                         dw, G->d_rp, G->d_adj, indeg.as<int32_t>(),
-                                                        di + 2, (unsigned long long*)(di + 4), di + 1);
+                                                        di + 2, (unsigned long long*)(di + 4), di + 6, di + 1);
     fbc::gb_max_kernel<<<grid_for(n), 256, 0, g.st>>>(n, indeg.as<int32_t>(), di + 3);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(hi, ints.p, sizeof(hi), cudaMemcpyDeviceToHost, g.st);
@@ -1247,6 +1451,7 @@ int device_csr_build(int64_t count, const int32_t* dsrc, const int32_t* ddst, co
     G->m = medges;
     G->maxw = hi[2];
     G->maxindeg = hi[3];
+    G->maxdeg = hi[6];
     G->meanw = medges ? (double)sumw / (double)medges : 1.0;
     if ((double)n * (double)G->maxw > 2147483646.0) {
         drop();
@@ -1409,7 +1614,7 @@ int fbc_gpu_shutdown(void) {
     cudaStreamSynchronize(g.st);
     for (DBuf* b : {&g.c_off, &g.c_id, &g.c_lid, &g.c_isb, &g.c_flag, &g.c_scan, &g.c_sums, &g.c_boff,
                     &g.c_bsrc, &g.c_m, &g.c_err, &g.retry, &g.segs, &g.units_b, &g.units_w, &g.chunks, &g.crp, &g.cadj, &g.cgid, &g.cbord, &g.bc,
-                    &g.bdist, &g.bsig, &g.ctr, &g.dbg})
+                    &g.bdist, &g.bsig, &g.ctr, &g.dbg, &g.bcseg, &g.tsegs, &g.tquad, &g.textra, &g.tunits, &g.tchunks})
         b->release();
     g.wsb.buf.release();
     g.wsw.buf.release();
@@ -1707,6 +1912,7 @@ int fbc_exact_bc(fbc_graph G, int precision, int sched, double* out_bc, fbc_stat
     P.seg_m.push_back(G->m);
     P.seg_maxw.push_back(G->maxw);
     P.seg_maxindeg.push_back(G->maxindeg);
+    P.seg_maxdeg.push_back(G->maxdeg);
     for (int32_t s = 0; s < G->n; ++s) P.units.push_back(Unit{0, s, 1.0, -1});
     P.bc_len = G->n;
     FBC_TRY(run_plan(P, st));
@@ -1738,6 +1944,7 @@ int fbc_sssp_dependency_batch(fbc_graph G, int64_t count, const int32_t* sources
     P.seg_m.push_back(G->m);
     P.seg_maxw.push_back(G->maxw);
     P.seg_maxindeg.push_back(G->maxindeg);
+    P.seg_maxdeg.push_back(G->maxdeg);
     for (int64_t i = 0; i < count; ++i)
         P.units.push_back(Unit{0, map ? map[sources[i]] : sources[i], cards ? cards[i] : 1.0, -1});
     // on a relabelled graph, sources in the locality order: the sources running at once then
@@ -2070,10 +2277,12 @@ namespace {
 // uncaptured: fbc_plan_run then takes the general path.
 template <class Prec>
 int plan_capture(fbc_plan_s* p, Plan& P) {
-    std::vector<char> small(P.segs.size(), 0);
-    for (size_t s = 0; s < P.segs.size(); ++s)
-        small[s] = P.segs[s].n <= std::min<int64_t>(g.opt.warp_max_n, 65535) && P.seg_maxw[s] < 65536 &&
-                   P.seg_m[s] < ((int64_t)1 << 30);
+    std::vector<char> small(P.segs.size(), 0), team(P.segs.size(), 0);
+    for (size_t s = 0; s < P.segs.size(); ++s) {
+        const bool up_to = P.segs[s].n <= std::min<int64_t>(g.opt.warp_max_n, 65535);
+        team[s] = (up_to || team_takes_blocks()) && team_fits(P, s);
+        small[s] = !team[s] && up_to && P.seg_maxw[s] < 65536 && P.seg_m[s] < ((int64_t)1 << 30);
+    }
     for (;;) {  // the shared-memory layout fits at least two warps of the largest small segment
         int nm = 0, mm = 0, arg = -1;
         for (size_t s = 0; s < P.segs.size(); ++s)
@@ -2085,11 +2294,16 @@ int plan_capture(fbc_plan_s* p, Plan& P) {
         small[arg] = 0;
     }
     std::vector<std::vector<Unit>> by_seg(P.segs.size());
-    std::vector<Unit> uw, ub;
+    std::vector<Unit> uw, ub, ut[2];
     int nw_max = 0, mw_max = 0, nw_min = 1 << 30, nb_max = 0;
     for (const Unit& u : P.units) {
         const Seg& sg = P.segs[u.seg];
-        if (small[u.seg]) {
+        const bool up_to = small[u.seg] || (team[u.seg] && sg.n <= g.opt.warp_max_n);
+        (up_to ? p->wunits : p->bunits_n) += 1;
+        (up_to ? p->wbytes : p->bbytes) += 40.0 * (double)P.seg_m[u.seg] + 52.0 * sg.n;
+        if (team[u.seg]) {
+            ut[up_to ? 0 : 1].push_back(u);
+        } else if (small[u.seg]) {
             by_seg[u.seg].push_back(u);
             nw_max = std::max(nw_max, sg.n);
             nw_min = std::min(nw_min, sg.n);
@@ -2158,20 +2372,32 @@ int plan_capture(fbc_plan_s* p, Plan& P) {
         K.ws_stride = bc.stride;
         K.ws_n = (int32_t)(nb_max * bc.K);
     }
+    TeamCfg tc[2];
+    fbc::TeamParams T[2];
+    int nteam = 0;
+    for (int i = 0; i < 2; ++i) {
+        if (ut[i].empty()) continue;
+        ++nteam;
+        fbc_plan_s::Team& t = p->team[i];
+        team_config(P, std::move(ut[i]), tc[i]);
+        FBC_TRY(team_upload(tc[i], p->segs.as<Seg>(), t.segs, t.quad, t.extra, t.units, t.chunks, nullptr));
+        T[i] = team_params(tc[i], base, t.segs, t.extra, t.units, t.chunks, p->ctr.as<unsigned long long>() + 4 + i);
+        FBC_CK(cudaFuncSetAttribute(fbc::team_kernel<Prec>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T[i].smem));
+    }
     FBC_CK(cudaStreamSynchronize(g.st));
-    for (const Unit& u : uw) p->wbytes += 40.0 * (double)P.seg_m[u.seg] + 52.0 * P.segs[u.seg].n;
-    for (const Unit& u : ub) p->bbytes += 40.0 * (double)P.seg_m[u.seg] + 52.0 * P.segs[u.seg].n;
-    p->wunits = (int64_t)uw.size();
-    p->bunits_n = (int64_t)ub.size();
-    p->launches = (uw.empty() ? 0 : 1) + (ub.empty() ? 0 : 1);
+    p->launches = (uw.empty() ? 0 : 1) + (ub.empty() ? 0 : 1) + nteam;
     FBC_CK(cudaStreamBeginCapture(g.st, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(p->ctr.p, 0, 64, g.st);
     cudaMemsetAsync(p->bc.p, 0, n8, g.st);
     if (!uw.empty()) fbc::small_seg_kernel<Prec><<<(unsigned)cfg.blocks, 32 * cfg.wpb, (size_t)cfg.dyn, g.st>>>(S);
+    if (tc[0].blocks)
+        fbc::team_kernel<Prec><<<(unsigned)tc[0].blocks, fbc::kTeamThreads, (size_t)T[0].smem, g.st>>>(T[0]);
     cudaError_t ce = cudaStreamEndCapture(g.st, &p->graph[0]);
     if (ce != cudaSuccess) return fail(FBC_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(ce));
     FBC_CK(cudaGraphInstantiate(&p->exec[0], p->graph[0], 0));
     FBC_CK(cudaStreamBeginCapture(g.st, cudaStreamCaptureModeThreadLocal));
+    if (tc[1].blocks)
+        fbc::team_kernel<Prec><<<(unsigned)tc[1].blocks, fbc::kTeamThreads, (size_t)T[1].smem, g.st>>>(T[1]);
     if (!ub.empty()) launch_units(bc, K, g.st);
     cudaMemcpyAsync(p->h_bc, p->bc.p, n8, cudaMemcpyDeviceToHost, g.st);
     if (p->ent > 0) {
@@ -2313,6 +2539,7 @@ int fbc_multi_exact_bc(int32_t ngraphs, const fbc_graph* graphs, int precision, 
         P.seg_m.push_back(graphs[i]->m);
         P.seg_maxw.push_back(graphs[i]->maxw);
         P.seg_maxindeg.push_back(graphs[i]->maxindeg);
+        P.seg_maxdeg.push_back(graphs[i]->maxdeg);
         for (int32_t s = 0; s < graphs[i]->n; ++s) P.units.push_back(Unit{i, s, 1.0, -1});
         base[i + 1] = base[i] + graphs[i]->n;
     }
@@ -2342,6 +2569,7 @@ int fbc_sssp_debug(fbc_graph G, int32_t source, int32_t* out_dist, uint64_t* out
     P.seg_m.push_back(G->m);
     P.seg_maxw.push_back(G->maxw);
     P.seg_maxindeg.push_back(G->maxindeg);
+    P.seg_maxdeg.push_back(G->maxdeg);
     P.units.push_back(Unit{0, source, 1.0, -1});
     P.bc_len = G->n;
     P.dbg_sig = (unsigned long long*)base;

@@ -78,8 +78,8 @@ __global__ void gb_sort_rows_kernel(int32_t n, const int32_t* __restrict__ rs, u
 // merged rows: (dst, sum of its weights in input order) at rp[v] ..; per-graph statistics
 __global__ void gb_merge_kernel(int32_t n, const int32_t* __restrict__ rs, const unsigned long long* __restrict__ keys,
                                 const double* __restrict__ w, const int32_t* __restrict__ rp, int2* adj,
-                                int32_t* indeg, int* maxw, unsigned long long* sumw, int* err) {
-    int mw = 0;
+                                int32_t* indeg, int* maxw, unsigned long long* sumw, int* maxdeg, int* err) {
+    int mw = 0, md = 0;
     unsigned long long sw = 0;
     for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
         const int32_t a = rs[v], b = rs[v + 1];
@@ -98,11 +98,14 @@ __global__ void gb_merge_kernel(int32_t n, const int32_t* __restrict__ rs, const
             sw += (unsigned long long)wi;
             i = j;
         }
+        md = max(md, o - rp[v]);
     }
     mw = __reduce_max_sync(0xffffffffu, mw);
+    md = __reduce_max_sync(0xffffffffu, md);
     for (int d = 16; d > 0; d >>= 1) sw += __shfl_down_sync(0xffffffffu, sw, d);
     if ((threadIdx.x & 31) == 0) {
         atomicMax(maxw, mw);
+        atomicMax(maxdeg, md);
         atomicAdd(sumw, sw);  // one per warp: a per-thread add to one word serialises
     }
 }
