@@ -2023,9 +2023,9 @@ int fbc_kmeans(int32_t nsets, const int64_t* set_off, const int32_t* nb, const i
     const double t0 = now_ms();
     if (st) std::memset(st, 0, sizeof(*st));
     if (nsets == 0) return FBC_OK;
-    // sets, their points as (length, count) int pairs transposed per set (border-major), work areas
     std::vector<fbc::KMSet> sets((size_t)nsets);
     int64_t xs = 0, ws = 0, outs = 0;
+    double work = 0, most = 0;
     for (int32_t s = 0; s < nsets; ++s) {
         const int64_t np = set_off[s + 1] - set_off[s];
         if (np <= 0 || np > 0x7fffffff || nb[s] < 0 || k[s] < 1 || k[s] > np)
@@ -2035,6 +2035,8 @@ int fbc_kmeans(int32_t nsets, const int64_t* set_off, const int32_t* nb, const i
         S.np = (int32_t)np;
         S.nb = nb[s];
         S.k = k[s];
+        S.id = s;
+        S.in_off = xs;
         S.x_off = xs;
         S.ws_off = ws;
         S.out_off = outs;
@@ -2042,57 +2044,87 @@ int fbc_kmeans(int32_t nsets, const int64_t* set_off, const int32_t* nb, const i
         xs += np * nb[s];
         ws += fbc::km_work_bytes(np, nb[s], k[s]);
         outs += k[s];
+        const double w = (double)np * (nb[s] + 8.0);
+        work += w;
+        most = std::max(most, w);
     }
-    std::vector<int2> X((size_t)std::max<int64_t>(xs, 1));
-    for (int32_t s = 0; s < nsets; ++s) {
-        const fbc::KMSet& S = sets[(size_t)s];
-        double lmax = 0.0, cmax = 0.0;
-        for (int64_t j = 0; j < S.np; ++j)
-            for (int32_t i = 0; i < S.nb; ++i) {
-                const double l = len[vec_off[s] + j * S.nb + i];
-                const int32_t c = cnt[vec_off[s] + j * S.nb + i];
-                if (!(l >= 0.0 && l <= 2147483647.0) || l != std::floor(l))
-                    return fail(FBC_ERR_INVALID_ARG, "lengths must be integers in [0, 2^31)");
-                lmax = std::max(lmax, l);
-                cmax = std::max(cmax, std::fabs((double)c));
-                X[(size_t)(S.x_off + (int64_t)i * S.np + j)] = make_int2((int32_t)l, c);
-            }
-        // every squared distance exact in a double, as the reference's sums are on these inputs
-        if ((double)S.nb * (lmax * lmax + 4.0 * cmax * cmax) >= 9007199254740992.0)
-            return fail(FBC_ERR_RANGE, "set " + std::to_string(s) + ": squared distances may exceed 2^53");
-    }
-    TmpBuf dsets, dx, dwt, dws, didx, dw;
+    // blocks per set: as many as keep the GPU's two blocks per SM in use when the largest set is one of
+    // many, up to eight
+    int cluster = 1;
+    while (cluster < fbc::kKmCluster && 2 * cluster * work <= 2.0 * g.nsm * most) cluster *= 2;
+    std::vector<fbc::KMSet> order(sets);  // the largest first
+    std::stable_sort(order.begin(), order.end(), [](const fbc::KMSet& a, const fbc::KMSet& b) {
+        return (double)a.np * a.nb * a.k > (double)b.np * b.nb * b.k;
+    });
+    TmpBuf dsets, dlen, dcnt, dx, dmeta, dwt, dws, dout;
+    const size_t nx = (size_t)std::max<int64_t>(xs, 1);
     FBC_CK(dsets.ensure(sizeof(fbc::KMSet) * sets.size()));
-    FBC_CK(dx.ensure(sizeof(int2) * X.size()));
+    FBC_CK(dlen.ensure(sizeof(double) * nx));
+    FBC_CK(dcnt.ensure(sizeof(int32_t) * nx));
+    FBC_CK(dx.ensure(sizeof(int2) * nx));
+    FBC_CK(dmeta.ensure(sizeof(fbc::KMMeta) * sets.size(), true));
     FBC_CK(dwt.ensure(sizeof(int32_t) * (size_t)set_off[nsets]));
     FBC_CK(dws.ensure((size_t)std::max<int64_t>(ws, 256)));
-    FBC_CK(didx.ensure(sizeof(int32_t) * (size_t)outs));
-    FBC_CK(dw.ensure(sizeof(int32_t) * (size_t)outs));
-    FBC_CK(cudaMemcpyAsync(dsets.p, sets.data(), sizeof(fbc::KMSet) * sets.size(), cudaMemcpyHostToDevice, g.st));
-    FBC_CK(cudaMemcpyAsync(dx.p, X.data(), sizeof(int2) * X.size(), cudaMemcpyHostToDevice, g.st));
+    FBC_CK(dout.ensure(sizeof(int32_t) * 2 * (size_t)outs));
+    FBC_CK(cudaMemcpyAsync(dsets.p, order.data(), sizeof(fbc::KMSet) * order.size(), cudaMemcpyHostToDevice, g.st));
     FBC_CK(cudaMemcpyAsync(dwt.p, wt, sizeof(int32_t) * (size_t)set_off[nsets], cudaMemcpyHostToDevice, g.st));
+    for (int32_t s = 0; s < nsets;) {  // sets that lie back to back in the caller's arrays in one copy
+        int32_t e = s + 1;
+        while (e < nsets && vec_off[e] - vec_off[s] == sets[(size_t)e].in_off - sets[(size_t)s].in_off) ++e;
+        const int64_t o = sets[(size_t)s].in_off;
+        const size_t c = (size_t)((e < nsets ? sets[(size_t)e].in_off : xs) - o);
+        if (c > 0) {
+            FBC_CK(cudaMemcpyAsync(dlen.as<double>() + o, len + vec_off[s], sizeof(double) * c, cudaMemcpyHostToDevice, g.st));
+            FBC_CK(cudaMemcpyAsync(dcnt.as<int32_t>() + o, cnt + vec_off[s], sizeof(int32_t) * c, cudaMemcpyHostToDevice, g.st));
+        }
+        s = e;
+    }
     fbc::KMParams K{};
     K.sets = dsets.as<fbc::KMSet>();
+    K.meta = dmeta.as<fbc::KMMeta>();
     K.X = dx.as<int2>();
     K.wt = dwt.as<int32_t>();
     K.ws = dws.as<char>();
     K.min_variance = min_variance;
     K.max_iter = max_iter;
-    K.out_idx = didx.as<int32_t>();
-    K.out_w = dw.as<int32_t>();
+    K.out_idx = dout.as<int32_t>();
+    K.out_w = dout.as<int32_t>() + outs;
     FBC_CK(cudaEventRecord(g.ev0, g.st));
-    fbc::kmeans_kernel<<<(unsigned)nsets, 1024, 0, g.st>>>(K);
+    fbc::km_pack_kernel<<<dim3(64, (unsigned)std::min(nsets, 65535)), 256, 0, g.st>>>(
+        dsets.as<fbc::KMSet>(), nsets, dlen.as<double>(), dcnt.as<int32_t>(), dx.as<int2>(), dmeta.as<fbc::KMMeta>());
     FBC_CK(cudaGetLastError());
+    cudaLaunchConfig_t lc{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)cluster;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    lc.gridDim = dim3((unsigned)((int64_t)nsets * cluster));
+    lc.blockDim = dim3(fbc::kKmThreads);
+    lc.stream = g.st;
+    lc.attrs = &at;
+    lc.numAttrs = 1;
+    FBC_CK(cudaLaunchKernelEx(&lc, fbc::kmeans_kernel, K));
     FBC_CK(cudaEventRecord(g.ev1, g.st));
-    FBC_CK(cudaMemcpyAsync(out_idx, didx.p, sizeof(int32_t) * (size_t)outs, cudaMemcpyDeviceToHost, g.st));
-    FBC_CK(cudaMemcpyAsync(out_w, dw.p, sizeof(int32_t) * (size_t)outs, cudaMemcpyDeviceToHost, g.st));
+    std::vector<fbc::KMMeta> meta(sets.size());
+    std::vector<int32_t> res(2 * (size_t)outs);
+    FBC_CK(cudaMemcpyAsync(meta.data(), dmeta.p, sizeof(fbc::KMMeta) * meta.size(), cudaMemcpyDeviceToHost, g.st));
+    FBC_CK(cudaMemcpyAsync(res.data(), dout.p, sizeof(int32_t) * res.size(), cudaMemcpyDeviceToHost, g.st));
     FBC_CK(cudaStreamSynchronize(g.st));
+    for (int32_t s = 0; s < nsets; ++s) {
+        const fbc::KMMeta& m = meta[(size_t)s];
+        if (m.bad) return fail(FBC_ERR_INVALID_ARG, "lengths must be integers in [0, 2^31)");
+        // every squared distance exact in a double, as the reference's sums are on these inputs
+        if (fbc::km_range(nb[s], m.lmax, m.cmax) >= 9007199254740992.0)
+            return fail(FBC_ERR_RANGE, "set " + std::to_string(s) + ": squared distances may exceed 2^53");
+    }
+    std::copy(res.begin(), res.begin() + outs, out_idx);
+    std::copy(res.begin() + outs, res.end(), out_w);
     if (st) {
         float ms = 0.f;
         FBC_CK(cudaEventElapsedTime(&ms, g.ev0, g.ev1));
         st->kernel_ms = ms;
-        st->launches = 1;
-        st->h2d_bytes = (int64_t)(sizeof(int2) * X.size() + sizeof(int32_t) * set_off[nsets]);
+        st->launches = 2;
+        st->h2d_bytes = (int64_t)(12 * xs + sizeof(int32_t) * set_off[nsets]);
         st->d2h_bytes = (int64_t)(8 * outs);
         st->wall_ms = now_ms() - t0;
     }
