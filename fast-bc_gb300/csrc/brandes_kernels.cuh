@@ -55,6 +55,9 @@ struct Seg {
     int32_t n;              // vertices
     int32_t nb;             // border vertices (cluster segments), else 0
     int32_t delta;          // bucket width of the near-far pass
+    int32_t stamp_bits;     // log kernel: low bits of a word
+    const uint4* quad;      // log kernel: rows as quads of (destination:24 | weight:8)
+    int32_t wide;           // log kernel: rows of more than 8 edges
     int32_t pad;
 };
 

@@ -29,6 +29,7 @@
 #include "frontier_kernels.cuh"
 #include "kmeans.cuh"
 #include "team_kernels.cuh"
+#include "log_kernels.cuh"
 #include "host_order.hpp"
 
 namespace {
@@ -136,9 +137,11 @@ struct Ctx {
     DBuf retry, segs, units_b, units_w, chunks, crp, cadj, cgid, cbord, bc, bdist, bsig, ctr, dbg, bcseg;
     // team kernel: segment list, quads, continuation counts, units and work items of its launches
     DBuf tsegs, tquad, textra, tunits, tchunks;
+    // log kernel: quads of communities, the lists of a quad build, units
+    DBuf lquad, lsegs, lextra, lunits;
     // cluster extraction scratch: offsets, ids, flags, scans, given borders, error word
     DBuf c_off, c_id, c_lid, c_isb, c_flag, c_scan, c_sums, c_boff, c_bsrc, c_m, c_err;
-    Workspace wsb, wsw;
+    Workspace wsb, wsw, wsl;
 };
 Ctx g;
 
@@ -190,6 +193,8 @@ struct fbc_graph_s {
                                      // and weights are below 256
     int32_t* d_ord_inv = nullptr;
     std::vector<int32_t> ord_new;
+    // rows as quads (log kernel) of the input order and of the locality order, built on first use
+    uint4* d_quad[2] = {nullptr, nullptr};
 };
 
 struct fbc_plan_s {
@@ -197,6 +202,7 @@ struct fbc_plan_s {
     int prec = FBC_PREC_FP32C;
     int64_t n = 0, ent = 0;
     DBuf crp, cadj, cgid, cbord, segs, units, chunks, bc, bdist, bsig, ctr, retry, bunits, ws;
+    DBuf lquad, lsegs, lextra, lunits, lws;  // log launch
     struct Team {  // one team launch: communities up to warp_max_n, and above it
         DBuf segs, quad, extra, units, chunks;
     } team[2];
@@ -224,7 +230,7 @@ struct fbc_plan_s {
             if (graph[i]) cudaGraphDestroy(graph[i]);
         }
         for (DBuf* b : {&crp, &cadj, &cgid, &cbord, &segs, &units, &chunks, &bc, &bdist, &bsig, &ctr, &retry,
-                        &bunits, &ws})
+                        &bunits, &ws, &lquad, &lsegs, &lextra, &lunits, &lws})
             b->release();
         for (Team& t : team)
             for (DBuf* b : {&t.segs, &t.quad, &t.extra, &t.units, &t.chunks}) b->release();
@@ -327,6 +333,7 @@ struct Plan {
     std::vector<int32_t> seg_maxw;
     std::vector<int32_t> seg_maxindeg;
     std::vector<int32_t> seg_maxdeg;
+    std::vector<uint4**> seg_quads;  // where a whole graph keeps its quads (null: a community)
     std::vector<Unit> units;
     int64_t bc_len = 0;
     int64_t border_entries = 0;
@@ -475,7 +482,7 @@ int64_t ws_budget() {
     if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) return (int64_t)1 << 30;
     int64_t b = g.opt.ws_budget_mb > 0 ? g.opt.ws_budget_mb * (int64_t)1048576
                                         : (int64_t)((double)freeb * 0.6);
-    return b + (int64_t)g.wsb.buf.cap + (int64_t)g.wsw.buf.cap;
+    return b + (int64_t)g.wsb.buf.cap + (int64_t)g.wsw.buf.cap + (int64_t)g.wsl.buf.cap;
 }
 
 using KernFn = void (*)(fbc::KParams);
@@ -879,6 +886,178 @@ int launch_team(const Plan& P, std::vector<Unit>&& units, fbc_stats* st, int& la
     return FBC_OK;
 }
 
+// ---- log kernel (log_kernels.cuh): larger segments, one source per team in global memory ----
+
+// What its packed forms hold: 24-bit vertex and quad numbers, 8-bit weights, rows of up to 16 edges, 255
+// in-edges at most.  Tiny weights stay with the kernels of wider counts, as in team_fits.
+bool log_fits(const Plan& P, size_t s) {
+    const int64_t n = P.segs[s].n, maxw = P.seg_maxw[s];
+    return n >= 1 && P.seg_m[s] > 0 && P.seg_maxdeg[s] <= fbc::kLogRow && P.seg_maxindeg[s] <= fbc::kTeamIndeg &&
+           maxw >= kTeamMinMaxW && maxw < 256 && n + P.seg_m[s] / 3 + 1 < (int64_t)fbc::kQuadNone;
+}
+
+// Quads of the log kernel's segments: kept with a whole graph, else built into `quads`; the segment
+// list (already filled with them) is uploaded by the caller before the build kernels run.
+struct LogBuild {
+    std::vector<fbc::LogQuads> list;
+    std::vector<std::pair<uint4**, uint4*>> keep;  // a graph's, handed over once their build is launched
+    int nmax = 0;
+    ~LogBuild() {
+        for (auto& k : keep) cudaFree(k.second);
+    }
+};
+int log_quads_prepare(Plan& P, const std::vector<char>& logs, DBuf& quads, LogBuild& b) {
+    int64_t own = 0;
+    for (size_t s = 0; s < P.segs.size(); ++s)
+        if (logs[s] && !P.seg_quads[s]) own += P.segs[s].n + P.seg_m[s] / 3 + 1;
+    FBC_CK(quads.ensure(sizeof(uint4) * (size_t)std::max<int64_t>(own, 1)));
+    int64_t at = 0;
+    for (size_t s = 0; s < P.segs.size(); ++s) {
+        if (!logs[s]) continue;
+        Seg& sg = P.segs[s];
+        const int64_t nq = sg.n + P.seg_m[s] / 3 + 1;
+        uint4* q = nullptr;
+        bool build = true;
+        if (P.seg_quads[s]) {
+            q = *P.seg_quads[s];
+            for (auto& k : b.keep)  // the same graph twice in a batch
+                if (k.first == P.seg_quads[s]) q = k.second;
+            build = q == nullptr;
+            if (build) {
+                FBC_CK(cudaMalloc(&q, sizeof(uint4) * (size_t)nq));
+                b.keep.emplace_back(P.seg_quads[s], q);
+            }
+        } else {
+            q = quads.as<uint4>() + at;
+            at += nq;
+        }
+        sg.quad = q;
+        sg.wide = P.seg_maxdeg[s] > 8;
+        // stamp bits: what the distance bound leaves, or ten (then a source whose distances outgrow the
+        // others leaves the kernel)
+        sg.stamp_bits = std::min(24, std::max(fbc::kLogStamp, 32 - bit_length((uint64_t)sg.n * (uint64_t)P.seg_maxw[s] + 1)));
+        if (build) {
+            b.list.push_back(fbc::LogQuads{q, (int32_t)s, 0});
+            b.nmax = std::max(b.nmax, sg.n);
+        }
+    }
+    return FBC_OK;
+}
+int log_quads_build(LogBuild& b, const Seg* dsegs, DBuf& lsegs, DBuf& lextra, int& launches) {
+    if (b.list.empty()) return FBC_OK;
+    FBC_CK(lsegs.ensure(sizeof(fbc::LogQuads) * b.list.size()));
+    FBC_CK(lextra.ensure(sizeof(int32_t) * b.list.size()));
+    FBC_CK(cudaMemcpyAsync(lsegs.p, b.list.data(), sizeof(fbc::LogQuads) * b.list.size(), cudaMemcpyHostToDevice, g.st));
+    FBC_CK(cudaMemsetAsync(lextra.p, 0, sizeof(int32_t) * b.list.size(), g.st));
+    const dim3 grid((unsigned)b.list.size(), (unsigned)std::max(1, std::min(2048, (b.nmax + 255) / 256)));
+    fbc::log_quads_kernel<<<grid, 256, 0, g.st>>>(dsegs, lsegs.as<fbc::LogQuads>(), lextra.as<int32_t>());
+    FBC_CK(cudaGetLastError());
+    for (auto& k : b.keep) *k.first = k.second;
+    b.keep.clear();
+    ++launches;
+    return FBC_OK;
+}
+
+// Threads of a team and teams of a block.
+struct LogCfg {
+    KernFn kern = nullptr;
+    int threads = 0, teams = 0;
+    int64_t stride = 0, blocks = 0;
+    std::vector<Unit> units;  // biggest segments first
+};
+// 8, 4, 2 or 1 sources per SM (teams of 128, 256, 512, 1024 threads; four teams to a block of the
+// smallest).  More sources hide more latency, fewer leave each more of the L2: device time of the same
+// number of sources on road grids, relative to the best form of the size.
+int log_form(int64_t n, int64_t units) {
+    static const double at[5] = {20164, 65536, 262144, 1024000, 4194304};
+    static const double cost[5][4] = {{1.00, 1.28, 1.96, 3.55}, {1.00, 1.11, 1.52, 2.53}, {1.19, 1.00, 1.09, 1.56},
+                                      {1.56, 1.20, 1.00, 1.11}, {2.35, 1.49, 1.16, 1.00}};
+    int k = 0;
+    while (k < 3 && (double)n > at[k + 1]) ++k;
+    const double f = std::min(1.0, std::max(0.0, std::log((double)n / at[k]) / std::log(at[k + 1] / at[k])));
+    int best = 0;
+    double least = 0;
+    for (int i = 0; i < 4; ++i) {
+        // full waves, and a last one that takes somewhat less than half a wave's time at the least (a
+        // source with the SM to itself)
+        const double slots = (double)g.nsm * (8 >> i), waves = (double)units / slots, part = waves - std::floor(waves);
+        const double c = cost[k][i] + f * (cost[k + 1][i] - cost[k][i]);
+        const double t = c * slots * (std::floor(waves) + (part > 0 ? 0.45 + 0.55 * part : 0.0));
+        if (i == 0 || t < least) { best = i; least = t; }
+    }
+    return best;
+}
+template <class Prec>
+int log_config(const Plan& P, std::vector<Unit>&& units, int ws_n, int64_t budget, LogCfg& c) {
+    c = LogCfg{};
+    c.units = std::move(units);
+    std::stable_sort(c.units.begin(), c.units.end(), [&](const Unit& a, const Unit& b) {
+        const int na = P.segs[a.seg].n, nb = P.segs[b.seg].n;
+        return na != nb ? na > nb : a.seg < b.seg;
+    });
+    const int form = log_form((int64_t)ws_n, (int64_t)c.units.size());
+    const KernFn kern[4] = {fbc::log_kernel<Prec, 128, 4, 2>, fbc::log_kernel<Prec, 256, 1, 4>,
+                            fbc::log_kernel<Prec, 512, 1, 2>, fbc::log_kernel<Prec, 1024, 1, 1>};
+    c.kern = kern[form];
+    c.threads = 128 << form;
+    c.teams = form == 0 ? 4 : 1;
+    int bps = 1;
+    FBC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, c.kern, c.threads * c.teams, 0));
+    const int64_t sb = fbc::lstate_bytes<Prec>(ws_n);
+    c.stride = (sb + 255) & ~int64_t(255);
+    const int64_t want = std::min<int64_t>((int64_t)g.nsm * std::max(bps, 1), ((int64_t)c.units.size() + c.teams - 1) / c.teams);
+    c.blocks = std::max<int64_t>(1, std::min<int64_t>(want, budget / (c.stride * c.teams)));
+    return FBC_OK;
+}
+
+// A log-kernel launch on the library's workspace.
+template <class Prec>
+int launch_log(const Plan& P, std::vector<Unit>&& units, fbc_stats* st, int& launches) {
+    if (units.empty()) return FBC_OK;
+    int ws_n = 0;
+    for (const Unit& u : units) ws_n = std::max(ws_n, P.segs[u.seg].n);
+    LogCfg c;
+    FBC_TRY(log_config<Prec>(P, std::move(units), ws_n, ws_budget(), c));
+    Workspace& W = g.wsl;
+    if (!W.buf.p || (int64_t)W.buf.cap < c.blocks * c.teams * c.stride) {
+        W.buf.release();
+        FBC_CK(W.buf.ensure((size_t)(c.blocks * c.teams * c.stride)));
+    }
+    FBC_CK(g.lunits.ensure(sizeof(Unit) * c.units.size()));
+    FBC_CK(cudaMemcpyAsync(g.lunits.p, c.units.data(), sizeof(Unit) * c.units.size(), cudaMemcpyHostToDevice, g.st));
+    if (st) st->h2d_bytes += (int64_t)(sizeof(Unit) * c.units.size());
+    KParams K = base_params(P);
+    K.units = g.lunits.as<Unit>();
+    K.nunits = (int64_t)c.units.size();
+    K.next_unit = g.ctr.as<unsigned long long>() + 3;
+    K.ws = W.buf.as<char>();
+    K.ws_stride = c.stride;
+    K.ws_n = ws_n;
+    // one segment with an output map: BC is summed in the segment's order and scattered once at the end
+    const Seg& one = P.segs[c.units[0].seg];
+    bool single = one.gid != nullptr;
+    for (const Unit& u : c.units) single = single && u.seg == c.units[0].seg;
+    if (single) {
+        FBC_CK(g.bcseg.ensure(sizeof(double) * (size_t)one.n));
+        FBC_CK(cudaMemsetAsync(g.bcseg.p, 0, sizeof(double) * (size_t)one.n, g.st));
+        K.bc_seg = g.bcseg.as<double>();
+    }
+    c.kern<<<(unsigned)c.blocks, c.threads * c.teams, 0, g.st>>>(K);
+    FBC_CK(cudaGetLastError());
+    if (single) {
+        const unsigned gb = (unsigned)std::max<int64_t>(1, std::min<int64_t>((one.n + 255) / 256, 8192));
+        fbc::add_seg_kernel<<<gb, 256, 0, g.st>>>(K.bc_seg, one.gid, one.out_base, one.n, K.bc);
+        FBC_CK(cudaGetLastError());
+        ++launches;
+    }
+    ++launches;
+    if (st) {
+        st->slots = (int32_t)(c.blocks * c.teams);
+        st->group = c.teams;
+    }
+    return FBC_OK;
+}
+
 int map_err(int e) {
     if (e & fbc::kErrQueue) return fail(FBC_ERR_QUEUE, "device work queue overflow");
     if (e & fbc::kErrIter) return fail(FBC_ERR_ITER_LIMIT, "a device loop reached its iteration bound");
@@ -974,16 +1153,26 @@ int run_plan_t(Plan& P, fbc_stats* st) {
     // split units by kernel.  Batched: segments that fit the team kernel run there, up to
     // warp_max_n in one launch (with what the one-warp kernel takes, the first timed phase) and
     // above it in another; the rest run block-per-source.
-    std::vector<Unit> rest, tw, tb;
-    std::vector<char> team(P.segs.size(), 0);
+    std::vector<Unit> rest, tw, tb, lg;
+    std::vector<char> team(P.segs.size(), 0), logs(P.segs.size(), 0);
     if (P.sched == FBC_SCHED_BATCHED && !P.dbg_dist) {  // debug dumps come from block kernels
         const bool blocks = team_takes_blocks();
         for (size_t s = 0; s < P.segs.size(); ++s)
-            team[s] = (P.segs[s].n <= std::min<int64_t>(g.opt.warp_max_n, 65535) || blocks) && team_fits(P, s);
+        {
+            const bool up_to = P.segs[s].n <= std::min<int64_t>(g.opt.warp_max_n, 65535);
+            team[s] = (up_to || blocks) && team_fits(P, s);
+            logs[s] = !team[s] && !up_to && blocks && log_fits(P, s);
+        }
     }
     int64_t nwarp = 0, nblock = 0;  // units of the two phases
     double warp_bytes = 0, block_bytes = 0;
     for (const Unit& u : P.units) {
+        if (logs[u.seg]) {
+            lg.push_back(u);
+            nblock += 1;
+            block_bytes += 40.0 * (double)P.seg_m[u.seg] + 52.0 * P.segs[u.seg].n;
+            continue;
+        }
         if (!team[u.seg]) {
             rest.push_back(u);
             continue;
@@ -1001,6 +1190,8 @@ int run_plan_t(Plan& P, fbc_stats* st) {
     nblock += (int64_t)sp.ub.size();
     for (const Unit& u : sp.uw) warp_bytes += 40.0 * (double)P.seg_m[u.seg] + 52.0 * P.segs[u.seg].n;
     for (const Unit& u : sp.ub) block_bytes += 40.0 * (double)P.seg_m[u.seg] + 52.0 * P.segs[u.seg].n;
+    LogBuild lb;
+    if (!lg.empty()) FBC_TRY(log_quads_prepare(P, logs, g.lquad, lb));
     FBC_CK(g.segs.ensure(sizeof(Seg) * std::max<size_t>(P.segs.size(), 1)));
     FBC_CK(cudaMemcpyAsync(g.segs.p, P.segs.data(), sizeof(Seg) * P.segs.size(),
                            cudaMemcpyHostToDevice, g.st));
@@ -1015,6 +1206,8 @@ int run_plan_t(Plan& P, fbc_stats* st) {
         FBC_CK(cudaMemsetAsync(g.ctr.as<unsigned long long>() + 1, 0, 8, g.st));
         FBC_TRY(launch_team<Prec>(P, std::move(tb), st, launches));
     }
+    FBC_TRY(log_quads_build(lb, g.segs.as<Seg>(), g.lsegs, g.lextra, launches));
+    FBC_TRY(launch_log<Prec>(P, std::move(lg), st, launches));
     FBC_TRY(launch_old_blocks<Prec>(P, sp, st, launches));
     int err[2] = {0, 0};
     FBC_CK(cudaMemcpyAsync(err, (char*)g.ctr.p + 16, 2 * sizeof(int), cudaMemcpyDeviceToHost, g.st));
@@ -1321,6 +1514,7 @@ int prepare_clusters(const fbc_graph_s* G, int32_t nclusters, const int64_t* cof
         s.nb = (int32_t)(border_off[c + 1] - border_off[c]);
         s.delta = dl;
         P.segs.push_back(s);
+        P.seg_quads.push_back(nullptr);
         P.seg_m.push_back(seg_m[c]);
         P.seg_maxw.push_back(G->maxw);
         P.seg_maxindeg.push_back(G->maxindeg);
@@ -1614,12 +1808,14 @@ int fbc_gpu_shutdown(void) {
     cudaStreamSynchronize(g.st);
     for (DBuf* b : {&g.c_off, &g.c_id, &g.c_lid, &g.c_isb, &g.c_flag, &g.c_scan, &g.c_sums, &g.c_boff,
                     &g.c_bsrc, &g.c_m, &g.c_err, &g.retry, &g.segs, &g.units_b, &g.units_w, &g.chunks, &g.crp, &g.cadj, &g.cgid, &g.cbord, &g.bc,
-                    &g.bdist, &g.bsig, &g.ctr, &g.dbg, &g.bcseg, &g.tsegs, &g.tquad, &g.textra, &g.tunits, &g.tchunks})
+                    &g.bdist, &g.bsig, &g.ctr, &g.dbg, &g.bcseg, &g.tsegs, &g.tquad, &g.textra, &g.tunits, &g.tchunks, &g.lquad, &g.lsegs, &g.lextra, &g.lunits})
         b->release();
     g.wsb.buf.release();
     g.wsw.buf.release();
+    g.wsl.buf.release();
     g.wsb = Workspace();
     g.wsw = Workspace();
+    g.wsl = Workspace();
     cudaEventDestroy(g.ev0);
     cudaEventDestroy(g.ev1);
     cudaEventDestroy(g.evm);
@@ -1890,6 +2086,8 @@ int fbc_graph_free(fbc_graph G) {
     if (G->d_ord_adj4) cudaFree(G->d_ord_adj4);
     if (G->d_ord_revw) cudaFree(G->d_ord_revw);
     if (G->d_ord_inv) cudaFree(G->d_ord_inv);
+    for (uint4* q : G->d_quad)
+        if (q) cudaFree(q);
     delete G;
     return FBC_OK;
 }
@@ -1909,6 +2107,7 @@ int fbc_exact_bc(fbc_graph G, int precision, int sched, double* out_bc, fbc_stat
     const int32_t* map = nullptr;
     FBC_TRY(batched_graph_seg(G, 0, sched, sg, map));
     P.segs.push_back(sg);
+    P.seg_quads.push_back(&G->d_quad[map ? 1 : 0]);
     P.seg_m.push_back(G->m);
     P.seg_maxw.push_back(G->maxw);
     P.seg_maxindeg.push_back(G->maxindeg);
@@ -1941,6 +2140,7 @@ int fbc_sssp_dependency_batch(fbc_graph G, int64_t count, const int32_t* sources
     const int32_t* map = nullptr;
     FBC_TRY(batched_graph_seg(G, 0, sched, sg, map));
     P.segs.push_back(sg);
+    P.seg_quads.push_back(&G->d_quad[map ? 1 : 0]);
     P.seg_m.push_back(G->m);
     P.seg_maxw.push_back(G->maxw);
     P.seg_maxindeg.push_back(G->maxindeg);
@@ -2309,10 +2509,11 @@ namespace {
 // uncaptured: fbc_plan_run then takes the general path.
 template <class Prec>
 int plan_capture(fbc_plan_s* p, Plan& P) {
-    std::vector<char> small(P.segs.size(), 0), team(P.segs.size(), 0);
+    std::vector<char> small(P.segs.size(), 0), team(P.segs.size(), 0), logs(P.segs.size(), 0);
     for (size_t s = 0; s < P.segs.size(); ++s) {
         const bool up_to = P.segs[s].n <= std::min<int64_t>(g.opt.warp_max_n, 65535);
         team[s] = (up_to || team_takes_blocks()) && team_fits(P, s);
+        logs[s] = !team[s] && !up_to && P.segs[s].n <= 32768 && team_takes_blocks() && log_fits(P, s);
         small[s] = !team[s] && up_to && P.seg_maxw[s] < 65536 && P.seg_m[s] < ((int64_t)1 << 30);
     }
     for (;;) {  // the shared-memory layout fits at least two warps of the largest small segment
@@ -2326,14 +2527,16 @@ int plan_capture(fbc_plan_s* p, Plan& P) {
         small[arg] = 0;
     }
     std::vector<std::vector<Unit>> by_seg(P.segs.size());
-    std::vector<Unit> uw, ub, ut[2];
+    std::vector<Unit> uw, ub, ut[2], ul;
     int nw_max = 0, mw_max = 0, nw_min = 1 << 30, nb_max = 0;
     for (const Unit& u : P.units) {
         const Seg& sg = P.segs[u.seg];
         const bool up_to = small[u.seg] || (team[u.seg] && sg.n <= g.opt.warp_max_n);
         (up_to ? p->wunits : p->bunits_n) += 1;
         (up_to ? p->wbytes : p->bbytes) += 40.0 * (double)P.seg_m[u.seg] + 52.0 * sg.n;
-        if (team[u.seg]) {
+        if (logs[u.seg]) {
+            ul.push_back(u);
+        } else if (team[u.seg]) {
             ut[up_to ? 0 : 1].push_back(u);
         } else if (small[u.seg]) {
             by_seg[u.seg].push_back(u);
@@ -2356,6 +2559,8 @@ int plan_capture(fbc_plan_s* p, Plan& P) {
     FBC_CK(p->bsig.ensure(e8));
     FBC_CK(p->ctr.ensure(64));
     FBC_CK(p->retry.ensure(sizeof(fbc::RetryRec) * P.units.size()));
+    LogBuild lb;
+    if (!ul.empty()) FBC_TRY(log_quads_prepare(P, logs, p->lquad, lb));
     FBC_CK(cudaMemcpyAsync(p->segs.p, P.segs.data(), sizeof(Seg) * P.segs.size(), cudaMemcpyHostToDevice, g.st));
     KParams base{};
     base.segs = p->segs.as<Seg>();
@@ -2416,8 +2621,25 @@ int plan_capture(fbc_plan_s* p, Plan& P) {
         T[i] = team_params(tc[i], base, t.segs, t.extra, t.units, t.chunks, p->ctr.as<unsigned long long>() + 4 + i);
         FBC_CK(cudaFuncSetAttribute(fbc::team_kernel<Prec>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T[i].smem));
     }
+    LogCfg lc;
+    KParams L = base;
+    if (!ul.empty()) {
+        int quad_launches = 0, nl_max = 0;
+        for (const Unit& u : ul) nl_max = std::max(nl_max, P.segs[u.seg].n);
+        FBC_TRY(log_quads_build(lb, p->segs.as<Seg>(), p->lsegs, p->lextra, quad_launches));
+        FBC_TRY(log_config<Prec>(P, std::move(ul), nl_max, ws_budget(), lc));
+        FBC_CK(p->lunits.ensure(sizeof(Unit) * lc.units.size()));
+        FBC_CK(cudaMemcpyAsync(p->lunits.p, lc.units.data(), sizeof(Unit) * lc.units.size(), cudaMemcpyHostToDevice, g.st));
+        FBC_CK(p->lws.ensure((size_t)(lc.blocks * lc.teams * lc.stride)));
+        L.units = p->lunits.as<Unit>();
+        L.nunits = (int64_t)lc.units.size();
+        L.next_unit = p->ctr.as<unsigned long long>() + 3;
+        L.ws = p->lws.as<char>();
+        L.ws_stride = lc.stride;
+        L.ws_n = nl_max;
+    }
     FBC_CK(cudaStreamSynchronize(g.st));
-    p->launches = (uw.empty() ? 0 : 1) + (ub.empty() ? 0 : 1) + nteam;
+    p->launches = (uw.empty() ? 0 : 1) + (ub.empty() ? 0 : 1) + nteam + (lc.blocks ? 1 : 0);
     FBC_CK(cudaStreamBeginCapture(g.st, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(p->ctr.p, 0, 64, g.st);
     cudaMemsetAsync(p->bc.p, 0, n8, g.st);
@@ -2430,6 +2652,7 @@ int plan_capture(fbc_plan_s* p, Plan& P) {
     FBC_CK(cudaStreamBeginCapture(g.st, cudaStreamCaptureModeThreadLocal));
     if (tc[1].blocks)
         fbc::team_kernel<Prec><<<(unsigned)tc[1].blocks, fbc::kTeamThreads, (size_t)T[1].smem, g.st>>>(T[1]);
+    if (lc.blocks) lc.kern<<<(unsigned)lc.blocks, lc.threads * lc.teams, 0, g.st>>>(L);
     if (!ub.empty()) launch_units(bc, K, g.st);
     cudaMemcpyAsync(p->h_bc, p->bc.p, n8, cudaMemcpyDeviceToHost, g.st);
     if (p->ent > 0) {
@@ -2568,6 +2791,7 @@ int fbc_multi_exact_bc(int32_t ngraphs, const fbc_graph* graphs, int precision, 
         const int32_t* map = nullptr;
         FBC_TRY(batched_graph_seg(graphs[i], base[i], sched, sg, map));
         P.segs.push_back(sg);
+        P.seg_quads.push_back(&graphs[i]->d_quad[map ? 1 : 0]);
         P.seg_m.push_back(graphs[i]->m);
         P.seg_maxw.push_back(graphs[i]->maxw);
         P.seg_maxindeg.push_back(graphs[i]->maxindeg);
@@ -2598,6 +2822,7 @@ int fbc_sssp_debug(fbc_graph G, int32_t source, int32_t* out_dist, uint64_t* out
     P.prec = FBC_PREC_FP64;
     P.sched = (int)g.opt.debug_sched;
     P.segs.push_back(whole_graph_seg(G, 0));
+    P.seg_quads.push_back(nullptr);
     P.seg_m.push_back(G->m);
     P.seg_maxw.push_back(G->maxw);
     P.seg_maxindeg.push_back(G->maxindeg);
