@@ -759,16 +759,18 @@ int bit_length(uint64_t x) {
 
 // What the kernel's packed forms hold: 16-bit byte offsets of vertices, 16-bit quad numbers, 15-bit
 // weights, rows of up to 16 edges, 255 in-edges at most (sums of counts below 2^24), distances that
-// leave a word eight stamp bits; and two sources' state in a block's shared memory (with one, the
-// frontier kernel is faster: 47 against 55 ms for the sources of a 16,384-vertex grid).
+// leave a word eight stamp bits; and two sources' state in a block's shared memory.  With room for one the
+// log kernel is faster on many sources (34 against 55 ms for all those of a 16,384-vertex grid), but up to
+// about four an SM, where it runs half empty, the team kernel is (one source of that grid: 0.6
+// against 1.3 ms).
 // Graphs of tiny weights (kTeamMinMaxW) have many tied paths, whose counts outgrow the kernel's
 // on most sources: they stay with the kernels of wider counts.
 constexpr int64_t kTeamMinMaxW = 8;
-bool team_fits(const Plan& P, size_t s) {
+bool team_fits(const Plan& P, size_t s, int64_t units) {
     const int64_t n = P.segs[s].n, maxw = P.seg_maxw[s];
     return n >= 1 && n <= fbc::kTeamMaxN && P.seg_maxdeg[s] <= fbc::kTeamRow && P.seg_maxindeg[s] <= fbc::kTeamIndeg &&
            maxw >= kTeamMinMaxW && maxw < 32768 && bit_length((uint64_t)n * (uint64_t)maxw + 1) <= fbc::kTeamDistBits &&
-           n + P.seg_m[s] / 3 + 1 <= 65535 && 2 * fbc::team_bytes(n, P.seg_maxdeg[s] > 8) <= team_dyn_smem();
+           n + P.seg_m[s] / 3 + 1 <= 65535 && (units <= 4 * (int64_t)g.nsm ? 1 : 2) * fbc::team_bytes(n, P.seg_maxdeg[s] > 8) <= team_dyn_smem();
 }
 
 // Segments above warp_max_n go to the team kernel too, unless an option asks for the frontier
@@ -1160,7 +1162,7 @@ int run_plan_t(Plan& P, fbc_stats* st) {
         for (size_t s = 0; s < P.segs.size(); ++s)
         {
             const bool up_to = P.segs[s].n <= std::min<int64_t>(g.opt.warp_max_n, 65535);
-            team[s] = (up_to || blocks) && team_fits(P, s);
+            team[s] = (up_to || blocks) && team_fits(P, s, (int64_t)P.units.size());
             logs[s] = !team[s] && !up_to && blocks && log_fits(P, s);
         }
     }
@@ -2164,9 +2166,30 @@ int fbc_single_source(fbc_graph G, int32_t source, int precision, double* out_de
     DevGuard dg_;
     FBC_TRY(check_init(dg_));
     if (!G || !out_dep) return fail(FBC_ERR_INVALID_ARG, "null argument");
-    std::fill(out_dep, out_dep + G->n, 0.0);
-    const double one = 1.0;
-    return fbc_sssp_dependency_batch(G, 1, &source, &one, precision, FBC_SCHED_PLAIN, out_dep, st);
+    if (source < 0 || source >= G->n) {
+        if (st) std::memset(st, 0, sizeof(*st));
+        std::fill(out_dep, out_dep + G->n, 0.0);
+        return fail(FBC_ERR_INVALID_ARG, "source out of range");
+    }
+    const double t0 = now_ms();
+    if (st) std::memset(st, 0, sizeof(*st));
+    // One source: the team kernel's or the log kernel's threads on it, in the input order (the locality
+    // order costs more than one source gains), else the plain kernel.
+    Plan P;
+    P.prec = precision;
+    P.segs.push_back(whole_graph_seg(G, 0));
+    P.seg_quads.push_back(&G->d_quad[0]);
+    P.seg_m.push_back(G->m);
+    P.seg_maxw.push_back(G->maxw);
+    P.seg_maxindeg.push_back(G->maxindeg);
+    P.seg_maxdeg.push_back(G->maxdeg);
+    P.units.push_back(Unit{0, source, 1.0, -1});
+    P.bc_len = G->n;
+    P.sched = team_takes_blocks() && (team_fits(P, 0, 1) || log_fits(P, 0)) ? FBC_SCHED_BATCHED : FBC_SCHED_PLAIN;
+    FBC_TRY(run_plan(P, st));
+    FBC_TRY(download_bc(out_dep, G->n, false, st));
+    if (st) st->wall_ms = now_ms() - t0;
+    return FBC_OK;
 }
 
 int fbc_cluster_border_count(fbc_graph G, int32_t nclusters, const int64_t* coff,
@@ -2512,7 +2535,7 @@ int plan_capture(fbc_plan_s* p, Plan& P) {
     std::vector<char> small(P.segs.size(), 0), team(P.segs.size(), 0), logs(P.segs.size(), 0);
     for (size_t s = 0; s < P.segs.size(); ++s) {
         const bool up_to = P.segs[s].n <= std::min<int64_t>(g.opt.warp_max_n, 65535);
-        team[s] = (up_to || team_takes_blocks()) && team_fits(P, s);
+        team[s] = (up_to || team_takes_blocks()) && team_fits(P, s, (int64_t)P.units.size());
         logs[s] = !team[s] && !up_to && P.segs[s].n <= 32768 && team_takes_blocks() && log_fits(P, s);
         small[s] = !team[s] && up_to && P.seg_maxw[s] < 65536 && P.seg_m[s] < ((int64_t)1 << 30);
     }

@@ -109,3 +109,35 @@ def test_community_sizes_in_one_sweep(fg, prec, tol):
     for ev in (fg.cluster_eval_batch(g, cs, prec, fg.BATCHED), fg.ClusterPlan(g, cs, prec).run()):
         assert rel_err(ev.intra_bc, ref.intra_bc) <= tol
         assert np.array_equal(ev.border_dist, ref.border_dist) and np.array_equal(ev.border_sigma, ref.border_sigma)
+
+
+@pytest.mark.parametrize("rows,cols,counts", [(92, 95, (1, 40)), (128, 128, (1, 300, 620)), (129, 128, (1,))])
+def test_few_sources_of_larger_graphs(fg, rows, cols, counts):
+    """Up to four sources per SM run in shared memory with room for one source (8,700 to 16,384 vertices);
+    more, or a larger graph, in the log kernel.  Single sources, too."""
+    el = graphs.road_grid(rows, cols, seed=rows)
+    g, og = fg.Graph.from_edgelist(el), oracle.CSR.from_edgelist(el)
+    for count in counts:
+        src = np.arange(0, g.n, g.n // count, dtype=np.int32)[:count]
+        ref = oracle.exact_bc_sources(og, src, threads=8)
+        for prec, tol in FORMS:
+            st = fg.Stats()
+            assert rel_err(fg.dependency_batch(g, src, None, prec, fg.BATCHED, stats=st), ref) <= tol
+            assert (st.group == 0) == (g.n <= 16384 and count <= 608)
+            if count == 1:
+                assert rel_err(fg.single_source(g, 0, prec), ref) <= tol
+
+
+@pytest.mark.parametrize("prec,tol", FORMS)
+def test_single_source_forms(fg, prec, tol):
+    """A single source by the team kernel, the log kernel (input order) and, for rows too long for both, the
+    plain kernel; the source's own entry is 0; a bad source is refused."""
+    for el in (graphs.road_grid(20, 31, seed=2), graphs.road_grid(260, 270, seed=2), graphs.rgg_knn(3000, k=12, seed=21)):
+        g, og = fg.Graph.from_edgelist(el), oracle.CSR.from_edgelist(el)
+        for s in (0, el.n - 1):
+            got = fg.single_source(g, s, prec)
+            assert got[s] == 0 and rel_err(got, oracle.exact_bc_sources(og, np.array([s], np.int32))) <= tol
+        for s in (-1, el.n):
+            with pytest.raises(fg.FbcError) as e:
+                fg.single_source(g, s, prec)
+            assert e.value.code == fg.FBC_ERR_INVALID_ARG
