@@ -142,6 +142,8 @@ struct Ctx {
     // cluster extraction scratch: offsets, ids, flags, scans, given borders, error word
     DBuf c_off, c_id, c_lid, c_isb, c_flag, c_scan, c_sums, c_boff, c_bsrc, c_m, c_err;
     Workspace wsb, wsw, wsl;
+    void* stage = nullptr;  // page-locked
+    size_t stage_cap = 0;
 };
 Ctx g;
 
@@ -333,6 +335,7 @@ struct Plan {
     std::vector<int32_t> seg_maxw;
     std::vector<int32_t> seg_maxindeg;
     std::vector<int32_t> seg_maxdeg;
+    std::vector<std::pair<void*, size_t>> results;  // host memory that the call fills after the launches
     std::vector<uint4**> seg_quads;  // where a whole graph keeps its quads (null: a community)
     std::vector<Unit> units;
     int64_t bc_len = 0;
@@ -1211,6 +1214,7 @@ int run_plan_t(Plan& P, fbc_stats* st) {
     FBC_TRY(log_quads_build(lb, g.segs.as<Seg>(), g.lsegs, g.lextra, launches));
     FBC_TRY(launch_log<Prec>(P, std::move(lg), st, launches));
     FBC_TRY(launch_old_blocks<Prec>(P, sp, st, launches));
+    for (auto& r : P.results) fbc_host::prefault(r.first, r.second);  // while the kernels run
     int err[2] = {0, 0};
     FBC_CK(cudaMemcpyAsync(err, (char*)g.ctr.p + 16, 2 * sizeof(int), cudaMemcpyDeviceToHost, g.st));
     FBC_CK(cudaStreamSynchronize(g.st));
@@ -1284,11 +1288,26 @@ int check_sched(int sched) {
     return FBC_OK;
 }
 
+constexpr size_t kStageMax = (size_t)64 << 20;
+int ensure_stage(size_t bytes) {
+    if (g.stage && g.stage_cap >= bytes) return FBC_OK;
+    if (g.stage) cudaFreeHost(g.stage);
+    g.stage = nullptr;
+    g.stage_cap = 0;
+    FBC_CK(cudaMallocHost(&g.stage, std::max<size_t>(bytes, 1 << 20)));
+    g.stage_cap = std::max<size_t>(bytes, 1 << 20);
+    return FBC_OK;
+}
+
 int download_bc(double* out, int64_t len, bool accumulate, fbc_stats* st) {
     if (!out || len <= 0) return FBC_OK;
+    // what is added to the caller's array comes through page-locked memory (kept, up to kStageMax bytes)
     std::vector<double> tmp;
     double* dst = out;
-    if (accumulate) {
+    if (accumulate && sizeof(double) * (size_t)len <= kStageMax) {
+        FBC_TRY(ensure_stage(sizeof(double) * (size_t)len));
+        dst = (double*)g.stage;
+    } else if (accumulate) {
         tmp.resize((size_t)len);
         dst = tmp.data();
     }
@@ -1296,7 +1315,9 @@ int download_bc(double* out, int64_t len, bool accumulate, fbc_stats* st) {
     FBC_CK(cudaStreamSynchronize(g.st));
     if (st) st->d2h_bytes += (int64_t)(sizeof(double) * (size_t)len);
     if (accumulate)
-        for (int64_t i = 0; i < len; ++i) out[i] += tmp[(size_t)i];
+        fbc_host::host_parallel(len, [&](int64_t lo, int64_t hi) {
+            for (int64_t i = lo; i < hi; ++i) out[i] += dst[i];
+        }, 262144);
     return FBC_OK;
 }
 
@@ -1815,6 +1836,9 @@ int fbc_gpu_shutdown(void) {
     g.wsb.buf.release();
     g.wsw.buf.release();
     g.wsl.buf.release();
+    if (g.stage) cudaFreeHost(g.stage);
+    g.stage = nullptr;
+    g.stage_cap = 0;
     g.wsb = Workspace();
     g.wsw = Workspace();
     g.wsl = Workspace();
@@ -2048,6 +2072,24 @@ int fbc_graph_download(fbc_graph G, int64_t* row_ptr, int32_t* col, double* w) {
     if (!G) return fail(FBC_ERR_INVALID_ARG, "null graph");
     DevGuard dg_;
     FBC_TRY(check_init(dg_));
+    if (!G->host_ok && G->m > 0) {  // built on the device: converted there, copied into the caller's arrays
+        const size_t n1 = (size_t)G->n + 1, m = (size_t)G->m;
+        TmpBuf drp, dcol, dw;
+        FBC_CK(drp.ensure(sizeof(int64_t) * n1));
+        FBC_CK(dcol.ensure(sizeof(int32_t) * m));
+        FBC_CK(dw.ensure(sizeof(double) * m));
+        fbc::gb_export_kernel<<<grid_for(G->m), 256, 0, g.st>>>(G->n, G->m, G->d_rp, G->d_adj, drp.as<int64_t>(),
+                                                                dcol.as<int32_t>(), dw.as<double>());
+        FBC_CK(cudaGetLastError());
+        if (row_ptr) fbc_host::prefault(row_ptr, sizeof(int64_t) * n1);
+        if (col) fbc_host::prefault(col, sizeof(int32_t) * m);
+        if (w) fbc_host::prefault(w, sizeof(double) * m);
+        if (row_ptr) FBC_CK(cudaMemcpyAsync(row_ptr, drp.p, sizeof(int64_t) * n1, cudaMemcpyDeviceToHost, g.st));
+        if (col) FBC_CK(cudaMemcpyAsync(col, dcol.p, sizeof(int32_t) * m, cudaMemcpyDeviceToHost, g.st));
+        if (w) FBC_CK(cudaMemcpyAsync(w, dw.p, sizeof(double) * m, cudaMemcpyDeviceToHost, g.st));
+        FBC_CK(cudaStreamSynchronize(g.st));
+        return FBC_OK;
+    }
     FBC_TRY(ensure_host_csr(G));
     if (row_ptr) std::copy(G->h_rp.begin(), G->h_rp.end(), row_ptr);
     if (col) std::copy(G->h_col.begin(), G->h_col.end(), col);
@@ -2507,6 +2549,8 @@ int fbc_cluster_eval_batch(fbc_graph G, int32_t nclusters, const int64_t* coff,
     int64_t ent = 0;
     FBC_TRY(prepare_clusters(G, nclusters, coff, cverts, border_off, borders, precision, sched,
                              g.crp, g.cadj, g.cgid, g.cbord, P, ent, st));
+    if (out_bdist) P.results.emplace_back(out_bdist, sizeof(double) * (size_t)ent);
+    if (out_bsig) P.results.emplace_back(out_bsig, sizeof(uint64_t) * (size_t)ent);
     FBC_TRY(run_plan(P, st));
     FBC_TRY(download_bc(out_intra_bc, G->n, true, st));
     if (ent > 0 && (out_bdist || out_bsig)) {

@@ -19,6 +19,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+from concurrent.futures import ThreadPoolExecutor
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -114,6 +115,25 @@ def _ck(rc: int) -> None:
 
 def _ptr(a: np.ndarray | None):
     return None if a is None else a.ctypes.data_as(C.c_void_p)
+
+
+_COPIERS = min(16, os.cpu_count() or 1)
+_copy_pool: ThreadPoolExecutor | None = None
+
+
+def _copy(a: np.ndarray) -> np.ndarray:
+    """a.copy(), by several threads where it is large (the fresh pages' faults, not the bytes, take the
+    time of one; NumPy copies without the interpreter lock)."""
+    global _copy_pool
+    out = np.empty_like(a)
+    if a.nbytes < 8 << 20 or _COPIERS < 2:
+        out[:] = a
+        return out
+    if _copy_pool is None:
+        _copy_pool = ThreadPoolExecutor(_COPIERS)
+    cut = np.linspace(0, a.size, _COPIERS + 1).astype(np.int64)
+    list(_copy_pool.map(lambda k: np.copyto(out[cut[k]:cut[k + 1]], a[cut[k]:cut[k + 1]]), range(_COPIERS)))
+    return out
 
 
 _initialised = False
@@ -363,7 +383,7 @@ class ClusterPlan:
         bd = np.ctypeslib.as_array(C.cast(bdp, C.POINTER(C.c_double)), (max(e, 1),))[:e]
         bs = np.ctypeslib.as_array(C.cast(bsp, C.POINTER(C.c_uint64)), (max(e, 1),))[:e]
         if copy:
-            bc, bd, bs = bc.copy(), bd.copy(), bs.copy()
+            bc, bd, bs = _copy(bc), _copy(bd), _copy(bs)
         return ClusterEval(bc, bd, bs, self.cs, self.entry_off)
 
     def free(self) -> None:
