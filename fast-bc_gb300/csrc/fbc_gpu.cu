@@ -967,9 +967,48 @@ int log_quads_build(LogBuild& b, const Seg* dsegs, DBuf& lsegs, DBuf& lextra, in
 struct LogCfg {
     KernFn kern = nullptr;
     int threads = 0, teams = 0;
+    int cluster = 1;          // blocks of a source (log_cluster_kernel)
     int64_t stride = 0, blocks = 0;
     std::vector<Unit> units;  // biggest segments first
 };
+cudaError_t log_launch(const LogCfg& c, const KParams& K, cudaStream_t st) {
+    cudaLaunchConfig_t lc{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)c.cluster;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    lc.gridDim = dim3((unsigned)(c.blocks * c.cluster));
+    lc.blockDim = dim3((unsigned)(c.threads * c.teams));
+    lc.stream = st;
+    lc.attrs = &at;
+    lc.numAttrs = c.cluster > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&lc, c.kern, K);
+}
+
+// Blocks of a source: more where there are fewer sources than SMs, as far as the clusters all run at once.
+// An SM issues about one scattered access a clock, so a large source gains from several; a round then
+// costs two to three microseconds of barrier and counters in the first block's shared memory, which
+// smaller graphs' rounds do not make up for.  One source, 1, 2, 4 and 8 blocks: 65,536 vertices 3.2, 4.1,
+// 4.0, 4.0 ms; 262,144: 7.6, 8.0, 7.3, 7.2; 1.05M: 24.4, 22.2, 18.0, 16.7; 4.2M: 96, 73, 53, 44.
+constexpr int64_t kLogClusterN = 524288;
+int log_cluster(KernFn kern, int64_t n, int64_t units) {
+    int cluster = 1;
+    while (cluster < 8 && 2 * cluster * units <= (int64_t)g.nsm && n >= kLogClusterN) cluster *= 2;
+    for (; cluster > 1; cluster /= 2) {
+        cudaLaunchConfig_t lc{};
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)cluster;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        lc.gridDim = dim3((unsigned)(units * cluster));
+        lc.blockDim = dim3(1024);
+        lc.attrs = &at;
+        lc.numAttrs = 1;
+        int most = 0;
+        if (cudaOccupancyMaxActiveClusters(&most, kern, &lc) == cudaSuccess && most >= units) break;
+    }
+    return cluster;
+}
 // 8, 4, 2 or 1 sources per SM (teams of 128, 256, 512, 1024 threads; four teams to a block of the
 // smallest).  More sources hide more latency, fewer leave each more of the L2: device time of the same
 // number of sources on road grids, relative to the best form of the size.
@@ -1006,6 +1045,8 @@ int log_config(const Plan& P, std::vector<Unit>&& units, int ws_n, int64_t budge
     c.kern = kern[form];
     c.threads = 128 << form;
     c.teams = form == 0 ? 4 : 1;
+    if (form == 3) c.cluster = log_cluster(fbc::log_cluster_kernel<Prec>, ws_n, (int64_t)c.units.size());
+    if (c.cluster > 1) c.kern = fbc::log_cluster_kernel<Prec>;
     int bps = 1;
     FBC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, c.kern, c.threads * c.teams, 0));
     const int64_t sb = fbc::lstate_bytes<Prec>(ws_n);
@@ -1047,8 +1088,7 @@ int launch_log(const Plan& P, std::vector<Unit>&& units, fbc_stats* st, int& lau
         FBC_CK(cudaMemsetAsync(g.bcseg.p, 0, sizeof(double) * (size_t)one.n, g.st));
         K.bc_seg = g.bcseg.as<double>();
     }
-    c.kern<<<(unsigned)c.blocks, c.threads * c.teams, 0, g.st>>>(K);
-    FBC_CK(cudaGetLastError());
+    FBC_CK(log_launch(c, K, g.st));
     if (single) {
         const unsigned gb = (unsigned)std::max<int64_t>(1, std::min<int64_t>((one.n + 255) / 256, 8192));
         fbc::add_seg_kernel<<<gb, 256, 0, g.st>>>(K.bc_seg, one.gid, one.out_base, one.n, K.bc);
@@ -2719,7 +2759,7 @@ int plan_capture(fbc_plan_s* p, Plan& P) {
     FBC_CK(cudaStreamBeginCapture(g.st, cudaStreamCaptureModeThreadLocal));
     if (tc[1].blocks)
         fbc::team_kernel<Prec><<<(unsigned)tc[1].blocks, fbc::kTeamThreads, (size_t)T[1].smem, g.st>>>(T[1]);
-    if (lc.blocks) lc.kern<<<(unsigned)lc.blocks, lc.threads * lc.teams, 0, g.st>>>(L);
+    if (lc.blocks) log_launch(lc, L, g.st);
     if (!ub.empty()) launch_units(bc, K, g.st);
     cudaMemcpyAsync(p->h_bc, p->bc.p, n8, cudaMemcpyDeviceToHost, g.st);
     if (p->ent > 0) {

@@ -22,6 +22,7 @@
 // A source whose counts reach 2^24, whose distances outgrow a word, or with more rounds than are
 // kept stops before its dependencies and is done by the kernels with wider fields.
 #pragma once
+#include <cooperative_groups.h>
 #include "frontier_kernels.cuh"
 #include "team_kernels.cuh"
 
@@ -147,13 +148,28 @@ __device__ __forceinline__ void lpush(const bool (&want)[4], const uint32_t (&x)
     }
 }
 
-// One source by a team of kThreads threads; bar: its named barrier.
-template <class Prec, int kThreads>
+// A load of state that other threads of the source wrote: those of a cluster's other blocks are not in
+// this block's L1.
+template <bool kCluster, class T>
+__device__ __forceinline__ T lload(const T* p) {
+    if constexpr (kCluster) return __ldcg(p);
+    else return *p;
+}
+
+// One source by a team of kThreads threads (bar: its named barrier), or by the `threads` threads of a
+// cluster of blocks, whose control words lie in the first block's shared memory.  tid numbers the team's
+// threads, whole warps together.
+template <class Prec, int kThreads, bool kCluster = false>
 __device__ __forceinline__ void log_unit(const KParams& P, const Seg& sg, const Unit& u, const LState<Prec>& S, LogCtl& C,
-                                         int64_t cap, int tid, int bar) {
-    constexpr int nth = kThreads;
+                                         int64_t cap, int tid, int bar, int threads = kThreads) {
+    const int nth = kCluster ? threads : kThreads;
     const int n = sg.n, lane = tid & 31;
-    auto sync = [bar]() { asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(kThreads) : "memory"); };
+    auto sync = [bar]() {
+        if constexpr (kCluster)
+            asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        else
+            asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(kThreads) : "memory");
+    };
     const uint4* __restrict__ quads = sg.quad;
     const int sb = sg.stamp_bits;
     const uint32_t smask = (1u << sb) - 1u;
@@ -194,7 +210,7 @@ __device__ __forceinline__ void log_unit(const KParams& P, const Seg& sg, const 
                 for (int i = tid; i < n; i += nth) S.word[i] = __ldcg(S.word + i) | smask;
                 sync();
                 for (int i = tid; i < nfar; i += nth) {
-                    const uint32_t v = (fs ? S.far1 : S.far0)[i];
+                    const uint32_t v = lload<kCluster>((fs ? S.far1 : S.far0) + i);
                     S.word[v] = __ldcg(S.word + v) ^ 1u;  // listed once each
                 }
                 stamp = fst = smask - 1u;
@@ -217,7 +233,7 @@ __device__ __forceinline__ void log_unit(const KParams& P, const Seg& sg, const 
                 for (int b = s + (tid & ~31); b < e; b += nth) {
                     const int i = b + lane;
                     const bool act = i < e;
-                    const uint32_t v = S.log[act ? i : s];
+                    const uint32_t v = lload<kCluster>(S.log + (act ? i : s));
                     uint4 q = __ldg(quads + v);
                     const int dv = (int)(__ldcg(S.word + v) >> sb);  // may have dropped since the push
                     // only the last pop stays (an exchange: loading and storing the place separately made
@@ -272,7 +288,7 @@ __device__ __forceinline__ void log_unit(const KParams& P, const Seg& sg, const 
                 uint32_t* const qf = fs ? S.far0 : S.far1;
                 int dmin = kInf;
                 for (int i = tid; i < nfar; i += nth) {
-                    const int d = (int)(__ldcg(S.word + qo[i]) >> sb);
+                    const int d = (int)(__ldcg(S.word + lload<kCluster>(qo + i)) >> sb);
                     if (d >= T) dmin = min(dmin, d);
                 }
                 dmin = __reduce_min_sync(kFull, dmin);
@@ -287,7 +303,7 @@ __device__ __forceinline__ void log_unit(const KParams& P, const Seg& sg, const 
                 fst = --stamp;
                 for (int b = tid & ~31; b < nfar; b += nth) {
                     const int i = b + lane;
-                    const uint32_t x[4] = {i < nfar ? qo[i] : 0u, 0u, 0u, 0u};
+                    const uint32_t x[4] = {i < nfar ? lload<kCluster>(qo + i) : 0u, 0u, 0u, 0u};
                     const int d = i < nfar ? (int)(__ldcg(S.word + x[0]) >> sb) : -1;
                     const bool live = i < nfar && d >= Told;  // the far pile holds a vertex once per generation
                     const bool pn[4] = {live && d < T, false, false, false}, pf[4] = {live && d >= T, false, false, false};
@@ -327,7 +343,7 @@ __device__ __forceinline__ void log_unit(const KParams& P, const Seg& sg, const 
         if (tid == 0) S.sig[src] = 1u;
         sync();
         uint32_t high = 0u;
-        int s = 0, e = S.rnd[1];
+        int s = 0, e = lload<kCluster>(S.rnd + 1);
         // what a lane needs of its entry but the count: fixed by now, so the next round's is loaded
         // while this one ends (only the counts wait for the barrier)
         struct Pre {
@@ -336,21 +352,21 @@ __device__ __forceinline__ void log_unit(const KParams& P, const Seg& sg, const 
             uint32_t wv, wx[4];
         };
         auto load = [&](Pre& p, int i, int end) {
-            const uint32_t v = S.log[min(i, end - 1)];
+            const uint32_t v = lload<kCluster>(S.log + min(i, end - 1));
             const bool on = i < end && v != kNoEdge;
             p.v = on ? v : kNoEdge;
             p.q = on ? __ldg(quads + v) : none;
-            p.wv = on ? S.word[v] : 0u;
+            p.wv = on ? lload<kCluster>(S.word + v) : 0u;
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
                 const uint32_t a = quad_at(p.q, t);
-                p.wx[t] = (a >> 24) ? S.word[a & 0xffffffu] : kNoEdge;  // (final: the L1 may hold it)
+                p.wx[t] = (a >> 24) ? lload<kCluster>(S.word + (a & 0xffffffu)) : kNoEdge;  // (final: the L1 may hold it)
             }
         };
         Pre nx;
         load(nx, s + tid, e);
         for (int r = 0; r < nr; ++r) {
-            const int e2 = S.rnd[min(r + 2, nr)];
+            const int e2 = lload<kCluster>(S.rnd + min(r + 2, nr));
             for (int b = s + (tid & ~31); b < e; b += nth) {
                 const int i = b + lane;
                 if (b >= s + nth) load(nx, i, e);  // (a round wider than the team)
@@ -374,7 +390,7 @@ __device__ __forceinline__ void log_unit(const KParams& P, const Seg& sg, const 
 #pragma unroll
                     for (int t = 0; t < 4; ++t) {
                         const uint32_t a = quad_at(nx.q, t);
-                        nx.wx[t] = (a >> 24) ? S.word[a & 0xffffffu] : kNoEdge;
+                        nx.wx[t] = (a >> 24) ? lload<kCluster>(S.word + (a & 0xffffffu)) : kNoEdge;
                     }
                 }
                 if (i < e) S.ent[i] = on ? make_uint2(v | (mk << 24), sv) : make_uint2(kNoEdge, 1u);
@@ -398,24 +414,24 @@ __device__ __forceinline__ void log_unit(const KParams& P, const Seg& sg, const 
         const double card = u.card;
         double* const bc = P.bc_seg ? P.bc_seg : P.bc + sg.out_base;
         const int32_t* const gid = P.bc_seg ? nullptr : sg.gid;
-        int hi = total, lo = S.rnd[nr - 1];
+        int hi = total, lo = lload<kCluster>(S.rnd + nr - 1);
         struct Pre {  // an entry and its row, loaded a round ahead
             uint2 en;
             uint32_t m;
             uint4 q;
         };
         auto load = [&](Pre& p, int i, int end) {
-            p.en = i < end ? S.ent[i] : make_uint2(kNoEdge, 1u);
+            p.en = i < end ? lload<kCluster>(S.ent + i) : make_uint2(kNoEdge, 1u);
             const bool on = p.en.x != kNoEdge;
             const uint32_t v = p.en.x & 0xffffffu;
             p.m = on ? p.en.x >> 24 : 0u;
-            if (on && sg.wide) p.m |= (uint32_t)S.mhi[v] << 8;
+            if (on && sg.wide) p.m |= (uint32_t)lload<kCluster>(S.mhi + v) << 8;
             p.q = p.m ? __ldg(quads + v) : none;
         };
         Pre nx;
         load(nx, lo + tid, hi);
         for (int r = nr - 1; r >= 0; --r) {
-            const int lo2 = S.rnd[max(r - 1, 0)];
+            const int lo2 = lload<kCluster>(S.rnd + max(r - 1, 0));
             for (int b = lo + (tid & ~31); b < hi; b += nth) {
                 const int i = b + lane;
                 if (b >= lo + nth) load(nx, i, hi);
@@ -432,7 +448,7 @@ __device__ __forceinline__ void log_unit(const KParams& P, const Seg& sg, const 
 #pragma unroll
                         for (int t = 0; t < 4; ++t) {
                             const bool tight = ((m >> t) & 1u) && !(t == 3 && link);
-                            c[t] = tight ? S.coef[quad_at(nx.q, t) & 0xffffffu] : Prec::store(Prec::zero());
+                            c[t] = tight ? lload<kCluster>(S.coef + (quad_at(nx.q, t) & 0xffffffu)) : Prec::store(Prec::zero());
                         }
                         Prec::add_coefs(acc, c[0], c[1], c[2], c[3]);
                         if (!__any_sync(kFull, link)) break;
@@ -482,6 +498,28 @@ __global__ void __launch_bounds__(kThreads * kTeams, kPerSM) log_kernel(KParams 
         const Seg sg = P.segs[u.seg];
         log_unit<Prec, kThreads>(P, sg, u, S, C, P.ws_n, tid, team);  // (barriers inside)
     }
+}
+
+// One source per cluster of blocks: for fewer sources than the GPU has SMs.  A warp's neighbours in the
+// log go to different blocks, so that a round of a thousand vertices is spread over all of them.
+template <class Prec>
+__global__ void __launch_bounds__(1024, 1) log_cluster_kernel(KParams P) {
+    __shared__ LogCtl own;
+    auto cl = cooperative_groups::this_cluster();
+    const int nblk = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    LogCtl& C = *cl.map_shared_rank(&own, 0);
+    const int tid = (((int)threadIdx.x >> 5) * nblk + rank) * 32 + ((int)threadIdx.x & 31);
+    const LState<Prec> S = lstate_carve<Prec>(P.ws + (int64_t)(blockIdx.x / nblk) * P.ws_stride, P.ws_n);
+    for (;;) {
+        if (tid == 0) C.unit = (int)atomicAdd(P.next_unit, 1ull);
+        cl.sync();
+        const int ui = *(volatile int*)&C.unit;
+        if (ui >= P.nunits) break;
+        const Unit u = P.units[ui];
+        const Seg sg = P.segs[u.seg];
+        log_unit<Prec, 1024, true>(P, sg, u, S, C, P.ws_n, tid, 0, 1024 * nblk);
+    }
+    cl.sync();  // no block leaves while another may still read the first one's control words
 }
 
 }  // namespace fbc

@@ -87,3 +87,25 @@ def test_sources_that_leave(fg):
     b = np.concatenate([ids[:, 1:].ravel(), ids[1:].ravel()])
     g, og = _graph(fg, *_both(a, b, np.full(a.size, 9), np.full(a.size, 9)))
     _check(fg, g, og, 5, retries=True)
+
+
+@pytest.mark.parametrize("count", [1, 3, 60])
+def test_cluster_of_blocks(fg, count):
+    """Fewer sources than SMs of a graph of more than 524,288 vertices: several blocks to a source; the
+    single source in the input order, the batch in the locality order."""
+    el = graphs.road_grid(730, 740, seed=5)
+    g, og = fg.Graph.from_edgelist(el), oracle.CSR.from_edgelist(el)
+    _check(fg, g, og, count, retries=False)
+    if count == 1:
+        ref = oracle.exact_bc_sources(og, np.array([777], np.int32))
+        for prec, tol in FORMS:
+            assert rel_err(fg.single_source(g, 777, prec), ref) <= tol
+        old = fg.get_option("iter_mult")
+        fg.set_option("iter_mult", 0)
+        try:
+            with pytest.raises(fg.FbcError) as e:
+                fg.single_source(g, 777)
+            assert e.value.code == fg.FBC_ERR_ITER_LIMIT
+        finally:
+            fg.set_option("iter_mult", old)
+        assert rel_err(fg.single_source(g, 777), ref) <= FORMS[0][1]
