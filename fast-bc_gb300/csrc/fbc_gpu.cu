@@ -30,6 +30,7 @@
 #include "kmeans.cuh"
 #include "team_kernels.cuh"
 #include "log_kernels.cuh"
+#include "order_kernels.cuh"
 #include "host_order.hpp"
 
 namespace {
@@ -368,9 +369,18 @@ int ensure_host_csr(fbc_graph_s* G) {
     return FBC_OK;
 }
 
-// Build (once) the relabelled device CSR of a graph: rows ascending in the new ids.
+int order_on_device(fbc_graph_s* G, bool& done);
+
+// Build (once) the relabelled device CSR of a graph: rows ascending in the new ids.  On the device; on
+// the host where a row is too long for that or a part of the bisection takes too many rounds.
 int ensure_order(fbc_graph_s* G) {
     if (G->ord_built) return FBC_OK;
+    bool done = false;
+    FBC_TRY(order_on_device(G, done));
+    if (done) {
+        G->ord_built = true;
+        return FBC_OK;
+    }
     FBC_TRY(ensure_host_csr(G));
     const int32_t n = G->n;
     std::vector<int32_t> nw = fbc_host::bisection_order(n, G->h_rp, G->h_col, 16);
@@ -1832,6 +1842,106 @@ void tx_host_weights(const char* text, int64_t len, const std::vector<int2>& sl,
         stop = std::min(stop, ts[k]);
         bad_w = std::min(bad_w, tb[k]);
     }
+}
+
+// The locality order and the relabelled CSR, built by the device (order_kernels.cuh).  done = false: this
+// graph is one for the host.
+int order_on_device(fbc_graph_s* G, bool& done) {
+    done = false;
+    const int32_t n = G->n;
+    const auto drop = [&]() {
+        for (void** q : {(void**)&G->d_ord_rp, (void**)&G->d_ord_adj, (void**)&G->d_ord_inv, (void**)&G->d_ord_adj4,
+                         (void**)&G->d_ord_revw}) {
+            if (*q) cudaFree(*q);
+            *q = nullptr;
+        }
+    };
+    drop();  // what a call that ran out of memory left
+    if (n <= 0 || G->maxdeg > fbc::kOrdMaxDeg) return FBC_OK;
+    TmpBuf b0, b1, bm, bd, be;
+    const size_t ints = sizeof(int32_t) * (size_t)n;
+    FBC_CK(b0.ensure(ints));
+    FBC_CK(b1.ensure(ints));
+    FBC_CK(bm.ensure(ints));
+    FBC_CK(bd.ensure(ints));
+    FBC_CK(be.ensure(2 * sizeof(int32_t), true));
+    fbc::order_init_kernel<<<grid_for(n), 256, 0, g.st>>>(n, b0.as<int32_t>(), bm.as<int32_t>());
+    FBC_CK(cudaGetLastError());
+    fbc::OrderArgs A{};
+    A.rp = G->d_rp;
+    A.adj = G->d_adj;
+    A.ord = b0.as<int32_t>();
+    A.tmp = b1.as<int32_t>();
+    A.mark = bm.as<int32_t>();
+    A.err = be.as<int32_t>();
+    A.n = n;
+    int32_t* cur = b0.as<int32_t>();
+    int32_t* nxt = b1.as<int32_t>();
+    int32_t err[2] = {0, 0};
+    int level = 0;
+    int64_t parts = 1;
+    for (int64_t len = n; len > fbc::kOrdLeaf; len = (len + 1) / 2, ++level, parts *= 2) {
+        A.level = level;
+        A.parts = (int32_t)parts;
+        A.ord = cur;
+        A.tmp = nxt;
+        // threads: a BFS level of a road-like part is about sqrt(len) to twice that wide; a cluster while
+        // that is more than a block and the clusters of all parts fit the chip at once
+        const bool cluster = len > 131072 && parts * fbc::kOrdCluster <= g.nsm;
+        int threads = 32;
+        while (threads < 1024 && (int64_t)threads * threads < 4 * len) threads *= 2;
+        cudaLaunchConfig_t lc{};
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = fbc::kOrdCluster;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        lc.gridDim = dim3((unsigned)(cluster ? parts * fbc::kOrdCluster
+                                             : std::min<int64_t>(parts, (int64_t)g.nsm * (2048 / threads))));
+        lc.blockDim = dim3((unsigned)threads);
+        lc.stream = g.st;
+        lc.attrs = &at;
+        lc.numAttrs = cluster ? 1 : 0;
+        FBC_CK(cudaLaunchKernelEx(&lc, cluster ? fbc::order_split_kernel<true> : fbc::order_split_kernel<false>, A));
+        std::swap(cur, nxt);
+        if (level == 0) {  // the whole graph's BFS tells most of the graphs that the host should order
+            FBC_CK(cudaMemcpyAsync(err, be.p, sizeof(int32_t), cudaMemcpyDeviceToHost, g.st));
+            FBC_CK(cudaStreamSynchronize(g.st));
+            if (err[0]) return FBC_OK;
+        }
+    }
+    // the relabelled rows
+    int32_t* nw = bm.as<int32_t>();  // the marks are done with
+    const bool pack = n < (1 << 24) && G->maxw < 256, rev = G->maxw < 256;
+    const size_t m = (size_t)std::max<int64_t>(G->m, 1);
+    FBC_CK(cudaMalloc(&G->d_ord_rp, ints + sizeof(int32_t)));
+    FBC_CK(cudaMalloc(&G->d_ord_adj, sizeof(int2) * m));
+    FBC_CK(cudaMalloc(&G->d_ord_inv, ints));
+    if (pack) FBC_CK(cudaMalloc(&G->d_ord_adj4, sizeof(uint32_t) * m));
+    if (rev) FBC_CK(cudaMalloc(&G->d_ord_revw, m));
+    fbc::order_leaf_kernel<<<grid_for(parts), 256, 0, g.st>>>(n, level, (int32_t)parts, cur, G->d_ord_inv, nw);
+    fbc::order_degree_kernel<<<grid_for(n), 256, 0, g.st>>>(n, G->d_rp, G->d_ord_inv, bd.as<int32_t>());
+    FBC_CK(cudaGetLastError());
+    FBC_TRY(device_scan(bd.as<int32_t>(), n, G->d_ord_rp));
+    fbc::order_rows_kernel<<<grid_for(n), 256, 0, g.st>>>(n, G->d_rp, G->d_adj, G->d_ord_inv, nw, G->d_ord_rp,
+                                                         G->d_ord_adj, G->d_ord_adj4);
+    if (rev)
+        fbc::order_revw_kernel<<<grid_for(n), 256, 0, g.st>>>(n, G->d_ord_rp, G->d_ord_adj, G->d_ord_revw,
+                                                              be.as<int32_t>() + 1);
+    FBC_CK(cudaGetLastError());
+    G->ord_new.resize((size_t)n);
+    FBC_CK(cudaMemcpyAsync(G->ord_new.data(), nw, ints, cudaMemcpyDeviceToHost, g.st));
+    FBC_CK(cudaMemcpyAsync(err, be.p, sizeof(err), cudaMemcpyDeviceToHost, g.st));
+    FBC_CK(cudaStreamSynchronize(g.st));
+    if (rev && err[1]) {  // not symmetric
+        cudaFree(G->d_ord_revw);
+        G->d_ord_revw = nullptr;
+    }
+    if (err[0]) {
+        drop();
+        return FBC_OK;
+    }
+    done = true;
+    return FBC_OK;
 }
 
 }  // namespace

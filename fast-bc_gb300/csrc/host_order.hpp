@@ -1,6 +1,6 @@
 // Host helpers of the graph preparation: a chunked parallel loop on the host's threads and the
-// locality order (recursive BFS bisection) of batched runs on large graphs.  Plain C++ (no CUDA),
-// so the order can be tested on its own.
+// locality order (recursive BFS bisection) of batched runs on large graphs that the device does not
+// order itself.  Plain C++ (no CUDA), so the order can be tested on its own.
 #pragma once
 #include <algorithm>
 #include <atomic>
