@@ -2315,6 +2315,7 @@ int fbc_exact_bc(fbc_graph G, int precision, int sched, double* out_bc, fbc_stat
     P.seg_maxdeg.push_back(G->maxdeg);
     for (int32_t s = 0; s < G->n; ++s) P.units.push_back(Unit{0, s, 1.0, -1});
     P.bc_len = G->n;
+    P.results.emplace_back(out_bc, sizeof(double) * (size_t)G->n);
     FBC_TRY(run_plan(P, st));
     FBC_TRY(download_bc(out_bc, G->n, false, st));
     if (st) st->wall_ms = now_ms() - t0;
@@ -2354,6 +2355,7 @@ int fbc_sssp_dependency_batch(fbc_graph G, int64_t count, const int32_t* sources
         std::stable_sort(P.units.begin(), P.units.end(), [](const Unit& a, const Unit& b) { return a.src < b.src; });
     P.bc_len = G->n;
     if (st) st->h2d_bytes += count * (int64_t)(sizeof(int32_t) + sizeof(double));
+    P.results.emplace_back(out_bc_accum, sizeof(double) * (size_t)G->n);
     FBC_TRY(run_plan(P, st));
     FBC_TRY(download_bc(out_bc_accum, G->n, true, st));
     if (st) st->wall_ms = now_ms() - t0;
@@ -2385,6 +2387,7 @@ int fbc_single_source(fbc_graph G, int32_t source, int precision, double* out_de
     P.units.push_back(Unit{0, source, 1.0, -1});
     P.bc_len = G->n;
     P.sched = team_takes_blocks() && (team_fits(P, 0, 1) || log_fits(P, 0)) ? FBC_SCHED_BATCHED : FBC_SCHED_PLAIN;
+    P.results.emplace_back(out_dep, sizeof(double) * (size_t)G->n);
     FBC_TRY(run_plan(P, st));
     FBC_TRY(download_bc(out_dep, G->n, false, st));
     if (st) st->wall_ms = now_ms() - t0;
