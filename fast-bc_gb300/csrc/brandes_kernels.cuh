@@ -388,7 +388,7 @@ __device__ __forceinline__ void warp_push(bool want, int x, int* q, int* cnt, in
 // accesses and of its rounds: lane by lane four accesses are in flight instead of one, and the owner
 // search (ten shuffles a round) is gone.  All 6,390 sources of a 90 x 71 grid, FP64, blocks of 256:
 // 21.2 -> 13.5 ms; with one barrier a round instead of two and a division per vertex instead of one
-// per edge of the shortest-path DAG 10.8 ms; in blocks of 128 threads 8.0 ms.
+// per edge of the shortest-path DAG 10.8 ms; in blocks of 64 threads 7.3 ms.
 constexpr int kLaneRow = 16;
 
 // Warp-aggregated append of up to four values a lane (where want[t]) to q[0..cap), counter *cnt.

@@ -560,13 +560,17 @@ int block_config(const Plan& P, const std::vector<Unit>& units_in, int ws_n, boo
     int threads = (int)std::min<int64_t>(std::max<int64_t>(fr ? g.opt.frontier_threads : g.opt.block_threads, 32),
                                          fr ? 128 : 1024);
     if (wide) threads = (int)g.opt.wide_threads;
-    // plain schedule: a frontier of a segment of up to 32K vertices fills about 128 threads, so with
-    // units for eight such blocks an SM (as many as the registers allow) they beat four of 256
-    // (6,390 vertices, all sources: 8.0 against 10.8 ms; 20,164, 2,432 sources: 8.5 against 10.3;
-    // 65,536, 608 sources: 10.1 against 7.8; 64 threads: 7.2, 10.6 and 16 ms, with twice the state)
-    if (!fr && g.opt.block_threads == Options{}.block_threads && ws_n <= 32768 &&
-        (int64_t)units_in.size() >= 8 * (int64_t)g.nsm)
-        threads = 128;
+    // Plain schedule: registers allow four blocks of 256 threads an SM, eight of 128 or sixteen of 64, and
+    // the frontier of a segment of thousands of vertices does not fill 256.  So smaller blocks run where
+    // the larger ones of all units would not be resident at once: all sources of 1,225 vertices
+    // 0.94 ms with 256, 0.67 with 128, 0.55 with 64; of 6,390 10.9, 8.0 and 7.3; of 8,190 16.8, 12.1 and
+    // 12.2 (the state no longer pays); 900 sources on 20,164 vertices 5.0, 3.8 and 5.3, but 608 of them
+    // 2.8, 3.4 and 4.9; 608 on 65,536 7.8, 10.1 and 16.
+    if (!fr && g.opt.block_threads == Options{}.block_threads) {
+        const int64_t units = (int64_t)units_in.size();
+        if (ws_n <= 7168 && units > 8 * (int64_t)g.nsm) threads = 64;
+        else if (ws_n <= 32768 && units > 4 * (int64_t)g.nsm) threads = 128;
+    }
     threads = (threads / 32) * 32;
     // units sorted so that each segment's units are adjacent (the caller sorts by size)
     std::vector<Unit> sorted(units_in);

@@ -83,7 +83,7 @@ const char* fbc_last_error_string(void);
 /* Tuning knobs (the autotuner sets the first ones); values outside a knob's range are clamped:
  *   "delta"            bucket width of the distance pass (0 = 4 x the graph's mean weight)
  *   "block_threads"    block size of the plain kernel (32..1024; left at its default of 256, launches of many
- *                      sources on segments of up to 32,768 vertices take 128)
+ *                      sources on segments of up to 32,768 vertices take 128 or 64)
  *   "frontier_threads" block size of the frontier kernel (32..128; above 128 the wide form)
  *   "group"            sources per frontier block: 1, 2, 4, or 0 = automatic (others refused)
  *   "chunk_max"        sources per work item of the shared-memory kernel

@@ -1,7 +1,7 @@
 """The plain kernel's two ways over a warp's rows (each lane its own row when all 32 have at most 16
-edges, else the warp together) and its two block sizes: row lengths around a multiple of four and around
-16, rows of both kinds in one frontier, path counts that leave 64 bits, and the number of sources from
-which blocks of 128 threads run.  Against the oracle's exact BC."""
+edges, else the warp together) and its block sizes: row lengths around a multiple of four and around
+16, rows of both kinds in one frontier, path counts that leave 64 bits, and the numbers of sources above
+which smaller blocks run.  Against the oracle's exact BC."""
 import numpy as np
 import pytest
 
@@ -47,9 +47,9 @@ def test_one_long_row_among_short_ones(fg):
     _check(fg, g, og)
 
 
-@pytest.mark.parametrize("rows,cols", [(1, 2), (5, 13), (32, 38), (33, 37), (39, 40)])
+@pytest.mark.parametrize("rows,cols", [(1, 2), (5, 13), (19, 32), (21, 29), (32, 38), (33, 37), (39, 40)])
 def test_block_sizes(fg, rows, cols):
-    """1,216 sources (eight a multiprocessor) is where the blocks become smaller."""
+    """Above 608 and 1,216 sources (four and eight a multiprocessor) the blocks become smaller."""
     el = graphs.road_grid(rows, cols, seed=rows)
     _check(fg, fg.Graph.from_edgelist(el), oracle.CSR.from_edgelist(el))
 
