@@ -1,4 +1,5 @@
-// Batched schedule, small segments: a persistent kernel whose blocks pull (segment, chunk of
+// Batched schedule, small segments that the team kernel does not take (rows of more than 16 edges,
+// weights outside 8..32767, path counts from 2^24 on): a persistent kernel whose blocks pull (segment, chunk of
 // sources) work items from a queue; a block stages the segment's CSR in shared memory once
 // per chunk and each of its warps runs one source at a time with all per-source state in
 // shared memory as well, so the three Brandes passes read no global memory at all; only the

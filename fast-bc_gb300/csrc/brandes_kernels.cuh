@@ -99,6 +99,8 @@ struct KParams {
     int* retry_count;            // units to recompute one level up (null: report an error)
     RetryRec* retry;
     int32_t retry_cap;
+    int2* gave;                  // team and log kernels, per segment: units ended, units of these given
+                                 // back for wider counts (null: not counted)
     int32_t cnt_bits;            // frontier kernel: counter / mask bits next to the path count
     int32_t* dbg_dist;           // debug dump of one unit (may be null)
     unsigned long long* dbg_sig;
@@ -114,6 +116,20 @@ __device__ __forceinline__ void request_retry(const KParams& P, const Unit& u, i
     const int r = atomicAdd(P.retry_count, 1);
     if (r < P.retry_cap) P.retry[r] = RetryRec{u, code, 0};
     else atomicOr(P.err, kErrQueue);
+}
+
+// Units of a segment of which more than a third came back are handed back unstarted: a unit given back
+// has cost its distances and counts, about 0.6 of its time here, and is done again by a kernel that takes
+// a third longer, so with more than that it is better begun there.
+__device__ __forceinline__ bool gave_up(const KParams& P, int seg) {
+    if (!P.gave) return false;
+    const int2 c = __ldcg(P.gave + seg);
+    return c.x >= 16 && 3 * c.y > c.x;
+}
+__device__ __forceinline__ void count_unit(const KParams& P, int seg, bool back) {
+    if (!P.gave) return;
+    if (back) atomicAdd(&P.gave[seg].y, 1);
+    atomicAdd(&P.gave[seg].x, 1);
 }
 
 // ----------------------------------------------------------------------------- groups

@@ -140,6 +140,7 @@ struct Ctx {
     DBuf tsegs, tquad, textra, tunits, tchunks;
     // log kernel: quads of communities, the lists of a quad build, units
     DBuf lquad, lsegs, lextra, lunits;
+    DBuf gave;  // per segment: units ended, units given back
     // cluster extraction scratch: offsets, ids, flags, scans, given borders, error word
     DBuf c_off, c_id, c_lid, c_isb, c_flag, c_scan, c_sums, c_boff, c_bsrc, c_m, c_err;
     Workspace wsb, wsw, wsl;
@@ -460,6 +461,10 @@ Seg whole_graph_seg(const fbc_graph_s* G, int64_t out_base) {
     return s;
 }
 
+// Calls of at least this many units count the units that the team and log kernels give back (fewer are
+// begun at once).
+constexpr int64_t kCountUnits = 512;
+
 KParams base_params(const Plan& P) {
     KParams K{};
     K.segs = g.segs.as<Seg>();
@@ -471,6 +476,7 @@ KParams base_params(const Plan& P) {
     K.retry = g.retry.as<fbc::RetryRec>();
     K.retry_cap = (int32_t)(g.retry.cap / sizeof(fbc::RetryRec));
     K.iter_mult = (int32_t)g.opt.iter_mult;
+    K.gave = (int64_t)P.units.size() >= kCountUnits ? g.gave.as<int2>() : nullptr;
     K.dbg_dist = P.dbg_dist;
     K.dbg_sig = P.dbg_sig;
     K.dbg_dlt = P.dbg_dlt;
@@ -915,11 +921,16 @@ int launch_team(const Plan& P, std::vector<Unit>&& units, fbc_stats* st, int& la
 // ---- log kernel (log_kernels.cuh): larger segments, one source per team in global memory ----
 
 // What its packed forms hold: 24-bit vertex and quad numbers, 8-bit weights, rows of up to 16 edges, 255
-// in-edges at most.  Tiny weights stay with the kernels of wider counts, as in team_fits.
+// in-edges at most.  Tiny weights stay with the kernels of wider counts, as in team_fits, and so do small
+// ones on many vertices: the number of tied shortest paths grows with the hops (as the root of n) over the
+// weight.  Geometric graphs of weights up to 1000 / sqrt(n): 17 of 2,432 sources outgrow 24 bits at n = 16,384
+// (maxw 18), 1,268 at 24,000 (16), 2,293 at 32,000 (15); 24,000 vertices 27.4 ms here against 22.9, 12,000
+// 6.7 against 12.0.
 bool log_fits(const Plan& P, size_t s) {
     const int64_t n = P.segs[s].n, maxw = P.seg_maxw[s];
     return n >= 1 && P.seg_m[s] > 0 && P.seg_maxdeg[s] <= fbc::kLogRow && P.seg_maxindeg[s] <= fbc::kTeamIndeg &&
-           maxw >= kTeamMinMaxW && maxw < 256 && n + P.seg_m[s] / 3 + 1 < (int64_t)fbc::kQuadNone;
+           maxw >= kTeamMinMaxW && maxw < 256 && !(maxw < 32 && n > 74 * maxw * maxw) &&
+           n + P.seg_m[s] / 3 + 1 < (int64_t)fbc::kQuadNone;
 }
 
 // Quads of the log kernel's segments: kept with a whole graph, else built into `quads`; the segment
@@ -1214,6 +1225,10 @@ int run_plan_t(Plan& P, fbc_stats* st) {
     FBC_CK(g.bsig.ensure(sizeof(uint64_t) * std::max<int64_t>(P.border_entries, 1)));
     FBC_CK(g.ctr.ensure(64));
     FBC_CK(cudaMemsetAsync(g.ctr.p, 0, 64, g.st));
+    if ((int64_t)P.units.size() >= kCountUnits) {
+        FBC_CK(g.gave.ensure(sizeof(int2) * P.segs.size()));
+        FBC_CK(cudaMemsetAsync(g.gave.p, 0, sizeof(int2) * P.segs.size(), g.st));
+    }
     if (st) st->h2d_bytes += (int64_t)(sizeof(Seg) * P.segs.size());
 
     // split units by kernel.  Batched: segments that fit the team kernel run there, up to
@@ -1992,7 +2007,7 @@ int fbc_gpu_shutdown(void) {
     cudaStreamSynchronize(g.st);
     for (DBuf* b : {&g.c_off, &g.c_id, &g.c_lid, &g.c_isb, &g.c_flag, &g.c_scan, &g.c_sums, &g.c_boff,
                     &g.c_bsrc, &g.c_m, &g.c_err, &g.retry, &g.segs, &g.units_b, &g.units_w, &g.chunks, &g.crp, &g.cadj, &g.cgid, &g.cbord, &g.bc,
-                    &g.bdist, &g.bsig, &g.ctr, &g.dbg, &g.bcseg, &g.tsegs, &g.tquad, &g.textra, &g.tunits, &g.tchunks, &g.lquad, &g.lsegs, &g.lextra, &g.lunits})
+                    &g.bdist, &g.bsig, &g.ctr, &g.dbg, &g.bcseg, &g.tsegs, &g.tquad, &g.textra, &g.tunits, &g.tchunks, &g.lquad, &g.lsegs, &g.lextra, &g.lunits, &g.gave})
         b->release();
     g.wsb.buf.release();
     g.wsw.buf.release();
@@ -2733,10 +2748,10 @@ int fbc_cluster_eval_batch(fbc_graph G, int32_t nclusters, const int64_t* coff,
 
 namespace {
 // Capture of a prepared cluster sweep: counter and accumulator resets, the shared-memory kernel
-// for the communities that fit it, the frontier kernel (four sources per block) for the larger
-// ones on a workspace of the plan's own, and the downloads into pinned memory, as two CUDA graphs
-// replayed back to back (an event between them times the two kernels apart).  Communities that
-// need the plain kernels (above 32K vertices, in-degrees of 65,535 or more) leave the plan
+// for the communities that fit shared memory, the log kernel for the larger ones and the older kernels
+// for what these do not take, on workspaces of the plan's own, and the downloads into pinned memory, as
+// two CUDA graphs replayed back to back (an event between them times the two kernels apart).
+// Communities that need the plain kernels (above 32K vertices, in-degrees of 65,535 or more) leave the plan
 // uncaptured: fbc_plan_run then takes the general path.
 template <class Prec>
 int plan_capture(fbc_plan_s* p, Plan& P) {

@@ -1,5 +1,5 @@
 // Batched schedule, large segments (whole graphs: pivots, exact mode, big graphs of a
-// batch): one source (or a group of K sources) per thread block, per-source state in a
+// batch) that neither the team kernel nor the log kernel takes: one source (or a group of K sources) per thread block, per-source state in a
 // global-memory slot, blocks pulling units from a shared counter.  Same passes and predecessor
 // rule as brandes_kernels.cuh.  On million-vertex graphs the kernel is bound by random DRAM
 // sector accesses (every vertex's state and row is touched cold once per pass), so the

@@ -475,11 +475,24 @@ __device__ __forceinline__ void log_unit(const KParams& P, const Seg& sg, const 
             sync();
         }
     }
+    if (tid == 0) count_unit(P, u.seg, bad == kErrNarrow);
     if (bad && tid == 0) {
         if (bad == kErrNarrow) request_retry(P, u, kErrNarrow);  // recomputed with wider fields
         else atomicOr(P.err, bad);
     }
     sync();
+}
+
+// The next unit that is worth starting here; the others go back (one thread).
+__device__ __forceinline__ void log_pick(const KParams& P, LogCtl& C) {
+    for (;;) {
+        const int64_t ui = (int64_t)atomicAdd(P.next_unit, 1ull);
+        C.unit = (int)ui;
+        if (ui >= P.nunits) return;
+        const Unit u = P.units[ui];
+        if (!gave_up(P, u.seg)) return;
+        request_retry(P, u, kErrNarrow);
+    }
 }
 
 // kTeams teams of kThreads threads in a block, one source each.
@@ -490,7 +503,7 @@ __global__ void __launch_bounds__(kThreads * kTeams, kPerSM) log_kernel(KParams 
     LogCtl& C = ctl[team];
     const LState<Prec> S = lstate_carve<Prec>(P.ws + ((int64_t)blockIdx.x * kTeams + team) * P.ws_stride, P.ws_n);
     for (;;) {
-        if (tid == 0) C.unit = (int)atomicAdd(P.next_unit, 1ull);
+        if (tid == 0) log_pick(P, C);
         asm volatile("bar.sync %0, %1;" ::"r"(team), "n"(kThreads) : "memory");
         const int ui = *(volatile int*)&C.unit;
         if (ui >= P.nunits) break;
@@ -511,7 +524,7 @@ __global__ void __launch_bounds__(1024, 1) log_cluster_kernel(KParams P) {
     const int tid = (((int)threadIdx.x >> 5) * nblk + rank) * 32 + ((int)threadIdx.x & 31);
     const LState<Prec> S = lstate_carve<Prec>(P.ws + (int64_t)(blockIdx.x / nblk) * P.ws_stride, P.ws_n);
     for (;;) {
-        if (tid == 0) C.unit = (int)atomicAdd(P.next_unit, 1ull);
+        if (tid == 0) log_pick(P, C);
         cl.sync();
         const int ui = *(volatile int*)&C.unit;
         if (ui >= P.nunits) break;

@@ -521,6 +521,7 @@ __device__ __forceinline__ void TeamUnit<Prec, kWarp, kRows>::run(const KParams&
             sync();
         }
     }
+    if (tid == 0) count_unit(K, u.seg, bad == kErrNarrow);
     if (bad && tid == 0) {
         if (bad == kErrNarrow) request_retry(K, u, kErrNarrow);  // recomputed with wider counts
         else atomicOr(K.err, bad);
@@ -551,6 +552,17 @@ __device__ __forceinline__ TeamSplit team_split(int n, int nquads, bool wide, in
     t.W = max(1, min(nwarps / t.S, n >> 9));
     if (t.W > 1 && t.S > kTeamMax) t.W = 1;
     return t;
+}
+
+// The chunk's next unit that is worth starting here; the others go back (one thread).
+__device__ __forceinline__ int team_pick(const KParams& K, const Unit* units, int count, int* next) {
+    for (;;) {
+        const int k = atomicAdd(next, 1);
+        if (k >= count) return k;
+        const Unit u = units[k];
+        if (!gave_up(K, u.seg)) return k;
+        request_retry(K, u, kErrNarrow);
+    }
 }
 
 template <class Prec>
@@ -586,7 +598,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) team_kernel(TeamParams TP) {
                 int delta = team_delta(sg.delta);
                 for (;;) {
                     int k = 0;
-                    if (lane == 0) k = atomicAdd(&s_next, 1);
+                    if (lane == 0) k = team_pick(TP.k, units, ch.count, &s_next);
                     k = __shfl_sync(kFull, k, 0);
                     if (k >= ch.count) break;
                     if (sp.rows) U.run(TP.k, sg, units[k], ts, base, delta);
@@ -599,7 +611,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) team_kernel(TeamParams TP) {
                 TeamUnit<Prec, false, false> G{tid, sp.W * 32, lane, team + 1, ts.quad, C};
                 int delta = team_delta(sg.delta);
                 for (;;) {
-                    if (tid == 0) C->unit = atomicAdd(&s_next, 1);
+                    if (tid == 0) C->unit = team_pick(TP.k, units, ch.count, &s_next);
                     U.sync();
                     const int k = *(volatile int*)&C->unit;
                     if (k >= ch.count) break;

@@ -109,3 +109,34 @@ def test_cluster_of_blocks(fg, count):
         finally:
             fg.set_option("iter_mult", old)
         assert rel_err(fg.single_source(g, 777), ref) <= FORMS[0][1]
+
+
+@pytest.mark.parametrize("sources", [500, 511, 512, 1500])
+def test_units_given_back_unstarted(fg, sources):
+    """A grid of equal weights: nearly every source has 2^24 and more shortest paths somewhere, so from 512
+    sources on most are handed back without being begun."""
+    ids = np.arange(95 * 95).reshape(95, 95)
+    a = np.concatenate([ids[:, :-1].ravel(), ids[:-1].ravel()])
+    b = np.concatenate([ids[:, 1:].ravel(), ids[1:].ravel()])
+    g = fg.Graph.from_edges(np.concatenate([a, b]).astype(np.int32), np.concatenate([b, a]).astype(np.int32),
+                            np.full(2 * a.size, 40.0))
+    og = oracle.CSR(*g.csr())
+    src = np.linspace(0, ids.size - 1, sources).astype(np.int32)
+    ref = oracle.pivot_batch(og, src, np.ones(sources))
+    for prec, tol in FORMS:
+        st = fg.Stats()
+        assert rel_err(fg.dependency_batch(g, src, None, prec, fg.BATCHED, stats=st), ref) <= tol
+        assert st.retries >= sources
+
+
+def test_small_weights_on_many_vertices(fg):
+    """Weights below 32 on more than 74 * maxw^2 vertices start with the kernels of wider counts."""
+    el = graphs.rgg_knn(24000, seed=7, gid=3)
+    assert el.w.max() < 18
+    g, og = fg.Graph.from_edgelist(el), oracle.CSR.from_edgelist(el)
+    src = np.linspace(0, el.n - 1, 12).astype(np.int32)
+    ref = oracle.pivot_batch(og, src, np.ones(12))
+    for prec, tol in FORMS:
+        st = fg.Stats()
+        assert rel_err(fg.dependency_batch(g, src, None, prec, fg.BATCHED, stats=st), ref) <= tol
+        assert st.retries == 0
