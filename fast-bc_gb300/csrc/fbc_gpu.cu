@@ -222,6 +222,7 @@ struct fbc_plan_s {
     int launches = 0;
     std::vector<int64_t> coff, boff;
     std::vector<int32_t> cverts, borders;
+    std::vector<char> wide;  // communities whose counts outgrew the team or log kernel in a run
     // frees everything the plan holds, also when its creation stopped half way
     ~fbc_plan_s() {
         DevGuard dg_;
@@ -2758,8 +2759,9 @@ int plan_capture(fbc_plan_s* p, Plan& P) {
     std::vector<char> small(P.segs.size(), 0), team(P.segs.size(), 0), logs(P.segs.size(), 0);
     for (size_t s = 0; s < P.segs.size(); ++s) {
         const bool up_to = P.segs[s].n <= std::min<int64_t>(g.opt.warp_max_n, 65535);
-        team[s] = (up_to || team_takes_blocks()) && team_fits(P, s, (int64_t)P.units.size());
-        logs[s] = !team[s] && !up_to && P.segs[s].n <= 32768 && team_takes_blocks() && log_fits(P, s);
+        const bool packed = p->wide.empty() || !p->wide[s];
+        team[s] = packed && (up_to || team_takes_blocks()) && team_fits(P, s, (int64_t)P.units.size());
+        logs[s] = packed && !team[s] && !up_to && P.segs[s].n <= 32768 && team_takes_blocks() && log_fits(P, s);
         small[s] = !team[s] && up_to && P.seg_maxw[s] < 65536 && P.seg_m[s] < ((int64_t)1 << 30);
     }
     for (;;) {  // the shared-memory layout fits at least two warps of the largest small segment
@@ -2913,6 +2915,35 @@ int plan_capture(fbc_plan_s* p, Plan& P) {
     return FBC_OK;
 }
 
+// After a run in which communities' counts outgrew the team or log kernel: captured again with the kernels
+// of wider counts for these, so that the next run is a replay again.
+int plan_widen(fbc_plan_s* p) {
+    std::vector<fbc::RetryRec> rec((size_t)std::min<int64_t>(p->h_ctl[1], p->nunits));
+    FBC_CK(cudaMemcpy(rec.data(), p->retry.p, sizeof(fbc::RetryRec) * rec.size(), cudaMemcpyDeviceToHost));
+    p->wide.resize(p->coff.size(), 0);
+    bool more = false;
+    for (const fbc::RetryRec& r : rec)
+        if (r.code == fbc::kErrNarrow && !p->wide[r.u.seg]) {
+            p->wide[r.u.seg] = 1;
+            more = true;
+        }
+    if (!more) return FBC_OK;
+    for (int i = 0; i < 2; ++i) {
+        if (p->exec[i]) cudaGraphExecDestroy(p->exec[i]);
+        if (p->graph[i]) cudaGraphDestroy(p->graph[i]);
+        p->exec[i] = nullptr;
+        p->graph[i] = nullptr;
+    }
+    p->captured = false;
+    p->wbytes = p->bbytes = 0;
+    p->wunits = p->bunits_n = 0;
+    p->launches = 0;
+    Plan P;
+    FBC_TRY(prepare_clusters(p->G, (int32_t)p->coff.size() - 1, p->coff.data(), p->cverts.data(),
+                             p->boff.empty() ? nullptr : p->boff.data(), p->borders.empty() ? nullptr : p->borders.data(),
+                             p->prec, FBC_SCHED_BATCHED, p->crp, p->cadj, p->cgid, p->cbord, P, p->ent, nullptr));
+    return p->prec == FBC_PREC_FP64 ? plan_capture<fbc::PrecF64>(p, P) : plan_capture<fbc::PrecDF32>(p, P);
+}
 }  // namespace
 
 extern "C" {
@@ -2991,6 +3022,7 @@ int fbc_plan_run(fbc_plan p, fbc_stats* st) {
             return FBC_OK;
         }
         if (p->h_ctl[0] != 0 && p->h_ctl[1] == 0) return map_err(p->h_ctl[0]);
+        if (p->h_ctl[0] == 0 && plan_widen(p) != FBC_OK) (void)cudaGetLastError();  // stays on the general path
     }
     // not captured, or path counts needed a wider representation: the general path
     std::memset(p->h_bc, 0, sizeof(double) * (size_t)p->n);

@@ -64,15 +64,16 @@ typedef struct {
     double relaxations;      /* sum over units of the segment's edge count (TEPS numerator) */
     int32_t launches;        /* kernels launched by the call                               */
     int32_t slots;           /* concurrent block slots of the block-per-source kernel      */
-    double warp_ms;          /* device time of the warp-per-source kernel (CUDA events)    */
-    double block_ms;         /* device time of the block-per-source kernel (CUDA events)   */
-    double warp_bytes;       /* algorithmic bytes of the warp kernel's units               */
-    double block_bytes;      /* algorithmic bytes of the block kernel's units; one unit on a
+    double warp_ms;          /* device time of segments up to warp_max_n (CUDA events)     */
+    double block_ms;         /* device time of the larger ones (CUDA events)               */
+    double warp_bytes;       /* algorithmic bytes of the units up to warp_max_n            */
+    double block_bytes;      /* algorithmic bytes of the larger ones; one unit on a
                                 segment of n vertices and m edges counts 40*m + 52*n bytes  */
     int64_t warp_units;
     int64_t block_units;
-    int32_t group;           /* sources per block of the frontier kernel (0: not launched)  */
-    int32_t retries;         /* units recomputed by the plain kernel with wider path counts */
+    int32_t group;           /* sources per block of the log or the frontier kernel (0: neither launched) */
+    int32_t retries;         /* units recomputed by another kernel: path counts too wide for the first one,
+                                or more rounds than it keeps */
 } fbc_stats;
 
 /* Library lifetime.  fbc_gpu_init selects the device and creates the library stream. */
@@ -85,8 +86,12 @@ const char* fbc_last_error_string(void);
  *   "block_threads"    block size of the plain kernel (32..1024; left at its default of 256, launches of many
  *                      sources on segments of up to 32,768 vertices take 128 or 64)
  *   "frontier_threads" block size of the frontier kernel (32..128; above 128 the wide form)
- *   "group"            sources per frontier block: 1, 2, 4, or 0 = automatic (others refused)
- *   "chunk_max"        sources per work item of the shared-memory kernel
+ *                      (the frontier kernel runs what the team and log kernels do not take: rows of more
+ *                      than 16 edges, in-degrees above 255, weights outside 8..255 where the state is not
+ *                      in shared memory -- and everything above warp_max_n where "group" forces it)
+ *   "group"            0 = automatic; 1, 2, 4: segments above warp_max_n run on the frontier kernel with
+ *                      that many sources per block (others refused)
+ *   "chunk_max"        sources per work item of the shared-memory kernels
  *   "wide_n"           segments of at least this many vertices use the wide frontier blocks
  *   "wide_threads"     block size of the wide frontier blocks (64..1024, a multiple of 32; above 512
  *                      a 1024-thread form with 64 registers per thread; default 1024)
@@ -100,7 +105,9 @@ const char* fbc_last_error_string(void);
  *                      own row and the reverse weights, without atomics; 0: atomic counts
  *   "source_order"     1 (default): the sources of a batched call on a relabelled graph run in its
  *                      locality order (sources running at once start near each other); 0: as given
- *   "warp_max_n"       largest segment run warp-per-source in shared memory
+ *   "warp_max_n"       largest segment timed as "warp" in fbc_stats and run warp-per-source where the team
+ *                      kernel does not take it; 0 keeps every segment out of shared memory and off the
+ *                      team and log kernels
  *   "order_min_n"      batched runs relabel graphs of at least this many vertices for memory
  *                      locality (outputs stay in input ids)
  *   "csr_device_min_m" edge lists of at least this many edges are built into a CSR on the device
@@ -184,12 +191,13 @@ int fbc_cluster_eval_batch(fbc_graph g, int32_t nclusters, const int64_t* cluste
 
 /* Prepared cluster sweep for repeated evaluation of the same clusters (the Louvain-cluster
  * sweep of the clustered mode): the cluster subgraphs, units and work items are uploaded once
- * and the sweep (counter resets, the shared-memory kernel for the clusters that fit it, the
- * frontier kernel -- four sources per block, on a workspace of the plan's own -- for the larger
- * ones, downloads into pinned host buffers) is captured into CUDA graphs; fbc_plan_run replays
+ * and the sweep (counter resets, the team kernel for the clusters whose state fits shared memory, the
+ * log kernel for the larger ones and the older kernels for what these do not take, on workspaces of the
+ * plan's own, downloads into pinned host buffers) is captured into CUDA graphs; fbc_plan_run replays
  * them.  A plan with a cluster of more than 32,768 vertices (or a vertex of 65,535+ in-edges) is
  * not captured, and a run whose path counts need a wider representation is redone: both are
- * evaluated with fbc_cluster_eval_batch instead (same results).  fbc_plan_results gives host views of the
+ * evaluated with fbc_cluster_eval_batch instead (same results; after such a run the plan is captured again
+ * with kernels of wider counts for the clusters concerned).  fbc_plan_results gives host views of the
  * last run's intra-cluster BC (n entries, overwritten each run) and border vectors (layout of
  * fbc_cluster_eval_batch), valid until the next run or fbc_plan_free. */
 typedef struct fbc_plan_s* fbc_plan;
@@ -217,7 +225,7 @@ int fbc_cluster_classes(fbc_graph g, int32_t nclusters, const int64_t* cluster_o
 
 /* The k-means step of the clustered pivot selection (PlusPlusKMeans::computeCentroids,
  * PlusPlusKMeans.h:76-147, as KMeansPivotSelector.h:95-100 calls it) for nsets independent point
- * sets at once, one thread block each.  Set s has np_s = set_off[s+1] - set_off[s] points of
+ * sets at once, a cluster of up to eight thread blocks each.  Set s has np_s = set_off[s+1] - set_off[s] points of
  * nb[s] entries: point j's lengths len[vec_off[s] + j*nb[s] + i] (integers in [0, 2^31): a
  * normalized border vector, VertexInfo::normalize) and counts cnt[...] (the int border path counts
  * VertexInfo stores), weight wt[set_off[s] + j]; k[s] centroids (1 <= k <= np_s).  The reference's
