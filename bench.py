@@ -320,7 +320,7 @@ def run_clustered(args):
         mult[inp.clusters[c]] = float(np.sum(inp.cards[c]))
 
     # the batched form sweeps the communities as a prepared plan: subgraphs uploaded once, every
-    # step one replay of the captured CUDA graphs (shared-memory and frontier kernels)
+    # step one replay of the captured CUDA graphs (team and log kernels)
     plan, plan_ms = None, None
     if sched == fg.BATCHED:
         knobs("clusters")
@@ -411,10 +411,10 @@ def run_clustered(args):
     if os.path.exists(tpath) and dom == "block" and (prec, sched) == (fg.FP32C, fg.BATCHED):
         with open(tpath) as f:
             tw = json.load(f).get(args.workload)
-        if tw:  # the frontier-kernel launches of one step: ncu's DRAM bytes per source x sources
+        if tw:  # the log-kernel launches of one step: ncu's DRAM bytes per source x sources
             traffic = tw["pivot_bytes_per_unit"] * len(allp) + tw.get("sweep_block_bytes_per_unit", 0.0) * sweep_block_units
-    kname = {"block": "frontier_kernel (batched, block per source group)" if sched == fg.BATCHED
-             else "brandes_block_kernel", "warp": "small_seg_kernel (shared memory, warp per source)"}[dom]
+    kname = {"block": "log_kernel (batched, a team of warps per source, state in global memory)" if sched == fg.BATCHED
+             else "brandes_block_kernel", "warp": "team_kernel (a team of warps per source, state in shared memory)"}[dom]
     line = {"metric": METRIC, "value": value, "unit": "GTEPS", "n_gpus": ws, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": tot_dev / args.steps * 1e3,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
@@ -436,7 +436,7 @@ def run_clustered(args):
                          "frac": achieved / peak, "traffic": traffic, "kernel": kname,
                          "peak_source": peak_src,
                          "bytes_model": "40*m + 52*n per (segment, source) unit",
-                         "scope": "the frontier-kernel launches of one step (community sweep + pivots): achieved = "
+                         "scope": "the launches of one step on segments above warp_max_n (community sweep + pivots): achieved = "
                                   "their algorithmic bytes / their event time; traffic = ncu DRAM bytes per source "
                                   "x sources"},
             "clocks": clk}

@@ -5,7 +5,7 @@ size of the large-segment kernel (``frontier_threads``) and the number of source
 item of the shared-memory kernel (``chunk_max``) by timing candidates on a sample of the
 workload's units with the library's own CUDA events (``Stats.kernel_ms``).  Results only
 change speed, never values: every candidate computes the same distances, path counts and
-dependencies (the dependency sum is taken in adjacency order whatever the schedule).
+dependencies (a vertex's dependency is summed in adjacency order whatever the schedule).
 
     choice = autotune.tune_pivots(graph, sources, cards, fg.FP32C)      # applies and returns it
     choice = autotune.tune_clusters(graph, cluster_set, fg.FP32C)
@@ -83,8 +83,8 @@ def _tune_wide(g: fg.Graph, sources, cards, precision: int, sample: int,
 
 def tune_clusters(g: fg.Graph, cs: fg.ClusterSet, precision: int = fg.FP32C, sample: int = 16,
                   deltas=(2, 4, 8), chunks=(128, 512), threads=(128,)) -> dict:
-    """Cluster sources: delta, the shared-memory kernel's chunk size and (for clusters too large
-    for shared memory) the frontier kernel's block size, on a sample of the clusters (every k-th,
+    """Cluster sources: delta, the shared-memory kernels' chunk size and (for clusters that only the
+    frontier kernel takes) its block size, on a sample of the clusters (every k-th,
     keeping the size mix)."""
     cs = cs.with_borders(g)
     k = max(1, cs.count // sample)

@@ -350,8 +350,8 @@ def cluster_eval_batch(g: Graph, cs: ClusterSet, precision: int = FP64, sched: i
 
 class ClusterPlan:
     """A prepared cluster sweep (fbc_cluster_plan_create): the cluster subgraphs are uploaded
-    once and each run() replays captured CUDA graphs of the sweep's kernels (the shared-memory
-    kernel and/or the frontier kernel, by community size)."""
+    once and each run() replays captured CUDA graphs of the sweep's kernels (the team
+    kernel and/or the log kernel, by community size)."""
 
     def __init__(self, g: Graph, cs: ClusterSet, precision: int = FP64):
         self.g = g
