@@ -71,7 +71,7 @@ struct Unit {
 
 // A unit whose path counts outgrew the kernel's representation.  It stopped before its
 // dependency pass (nothing accumulated) and the host recomputes it one level up:
-// code kErrNarrow (team kernel) -> shared-memory or frontier kernel, kErrRetry -> plain kernel with
+// code kErrNarrow (team and log kernels) -> shared-memory or frontier kernel, kErrRetry -> plain kernel with
 // 64-bit counts, kErrSigma -> plain kernel with FP64
 // counts (the reference's own representation, exact below 2^53).
 struct RetryRec {

@@ -1880,10 +1880,11 @@ int order_on_device(fbc_graph_s* G, bool& done) {
     if (n <= 0 || G->maxdeg > fbc::kOrdMaxDeg) return FBC_OK;
     TmpBuf b0, b1, bm, bd, be;
     const size_t ints = sizeof(int32_t) * (size_t)n;
-    FBC_CK(b0.ensure(ints));
-    FBC_CK(b1.ensure(ints));
-    FBC_CK(bm.ensure(ints));
-    FBC_CK(bd.ensure(ints));
+    for (TmpBuf* b : {&b0, &b1, &bm, &bd})
+        if (b->ensure(ints) != cudaSuccess) {  // no scratch to be had: the host needs none
+            (void)cudaGetLastError();
+            return FBC_OK;
+        }
     FBC_CK(be.ensure(2 * sizeof(int32_t), true));
     fbc::order_init_kernel<<<grid_for(n), 256, 0, g.st>>>(n, b0.as<int32_t>(), bm.as<int32_t>());
     FBC_CK(cudaGetLastError());
