@@ -222,6 +222,7 @@ struct fbc_plan_s {
     int launches = 0;
     std::vector<int64_t> coff, boff;
     std::vector<int32_t> cverts, borders;
+    Options opt;             // as they were when the plan was made: a capture after a run follows them too
     std::vector<char> wide;  // communities whose counts outgrew the team or log kernel in a run
     // frees everything the plan holds, also when its creation stopped half way
     ~fbc_plan_s() {
@@ -2939,6 +2940,15 @@ int plan_widen(fbc_plan_s* p) {
     p->wbytes = p->bbytes = 0;
     p->wunits = p->bunits_n = 0;
     p->launches = 0;
+    // The new capture may lay the slots out differently (other communities, other free memory): the frontier
+    // kernel takes a slot whose header is not zero as one it has set up, so it starts from cleared ones again.
+    p->ws.release();
+    p->lws.release();
+    struct Restore {
+        Options now = g.opt;
+        ~Restore() { g.opt = now; }
+    } restore;
+    g.opt = p->opt;
     Plan P;
     FBC_TRY(prepare_clusters(p->G, (int32_t)p->coff.size() - 1, p->coff.data(), p->cverts.data(),
                              p->boff.empty() ? nullptr : p->boff.data(), p->borders.empty() ? nullptr : p->borders.data(),
@@ -2963,6 +2973,7 @@ int fbc_cluster_plan_create(fbc_graph G, int32_t nclusters, const int64_t* coff,
     p->G = G;
     p->prec = precision;
     p->n = G->n;
+    p->opt = g.opt;
     p->coff.assign(coff, coff + nclusters + 1);
     p->cverts.assign(cverts, cverts + coff[nclusters]);
     if (border_off) {
