@@ -1887,14 +1887,14 @@ int order_on_device(fbc_graph_s* G, bool& done) {
             return FBC_OK;
         }
     FBC_CK(be.ensure(2 * sizeof(int32_t), true));
-    fbc::order_init_kernel<<<grid_for(n), 256, 0, g.st>>>(n, b0.as<int32_t>(), bm.as<int32_t>());
+    fbc::order_init_kernel<<<grid_for(n), 256, 0, g.st>>>(n, b0.as<int32_t>(), bm.as<uint32_t>());
     FBC_CK(cudaGetLastError());
     fbc::OrderArgs A{};
     A.rp = G->d_rp;
     A.adj = G->d_adj;
     A.ord = b0.as<int32_t>();
     A.tmp = b1.as<int32_t>();
-    A.mark = bm.as<int32_t>();
+    A.mark = bm.as<uint32_t>();
     A.err = be.as<int32_t>();
     A.n = n;
     int32_t* cur = b0.as<int32_t>();
