@@ -485,25 +485,51 @@ KParams base_params(const Plan& P) {
     return K;
 }
 
+// Device memory that a launch on W may take for its slots (W null: a plan's own).  With ws_budget_mb all kept
+// workspaces share that many bytes; without, a launch may have 60% of what is free besides what W itself holds.
+int64_t ws_limit() { return g.opt.ws_budget_mb * (int64_t)1048576; }
+int64_t ws_budget(const Workspace* W) {
+    if (ws_limit() > 0) return ws_limit();
+    size_t freeb = 0, totalb = 0;
+    if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) return (int64_t)1 << 30;
+    return (int64_t)((double)freeb * 0.6) + (W ? (int64_t)W->buf.cap : 0);
+}
+
+// At least `bytes` in W (a new allocation cleared if `zero` is set).  The other kernels' workspaces are
+// idle between launches: they go where ws_budget_mb does not hold them beside W, or where there is no
+// memory for W otherwise.
+cudaError_t ws_take(Workspace& W, int64_t bytes, bool zero) {
+    const auto others = [&](int64_t keep) {
+        for (Workspace* o : {&g.wsb, &g.wsw, &g.wsl})
+            if (o != &W && (int64_t)(g.wsb.buf.cap + g.wsw.buf.cap + g.wsl.buf.cap - W.buf.cap) > keep) o->buf.release();
+    };
+    const int64_t limit = ws_limit();
+    if ((int64_t)W.buf.cap < bytes || (limit > 0 && (int64_t)W.buf.cap > std::max(limit, bytes))) W.buf.release();
+    if (limit > 0) others(std::max<int64_t>(0, limit - std::max(bytes, (int64_t)W.buf.cap)));
+    cudaError_t e = W.buf.ensure((size_t)bytes, zero, g.st);
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        others(0);
+        e = W.buf.ensure((size_t)bytes, zero, g.st);
+    }
+    return e;
+}
+
 // (Re)size a workspace for `slots` slots of at least `ws_n` vertices; reuse it when it
 // already fits (then the existing, possibly larger, capacity and stride are used).
 int ensure_ws(Workspace& W, int64_t slots, int64_t stride, int ws_n, int dsize) {
-    if (W.buf.p && W.ws_n >= ws_n && W.dsize == dsize && W.slots >= slots) return FBC_OK;
+    if (W.buf.p && W.ws_n >= ws_n && W.dsize == dsize && W.slots >= slots &&
+        !(ws_limit() > 0 && (int64_t)W.buf.cap > std::max(ws_limit(), slots * stride))) {
+        FBC_CK(ws_take(W, (int64_t)W.buf.cap, true));
+        return FBC_OK;
+    }
     W.buf.release();
-    FBC_CK(W.buf.ensure((size_t)(slots * stride), true, g.st));
+    FBC_CK(ws_take(W, slots * stride, true));
     W.stride = stride;
     W.slots = slots;
     W.ws_n = ws_n;
     W.dsize = dsize;
     return FBC_OK;
-}
-
-int64_t ws_budget() {
-    size_t freeb = 0, totalb = 0;
-    if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) return (int64_t)1 << 30;
-    int64_t b = g.opt.ws_budget_mb > 0 ? g.opt.ws_budget_mb * (int64_t)1048576
-                                        : (int64_t)((double)freeb * 0.6);
-    return b + (int64_t)g.wsb.buf.cap + (int64_t)g.wsw.buf.cap + (int64_t)g.wsl.buf.cap;
 }
 
 using KernFn = void (*)(fbc::KParams);
@@ -651,10 +677,10 @@ template <class Prec>
 int launch_block(const Plan& P, const std::vector<Unit>& units_in, int ws_n, fbc_stats* st,
                  int& launches, bool force_plain = false, bool sig_f64 = false) {
     if (units_in.empty()) return FBC_OK;
-    BlockCfg c;
-    FBC_TRY(block_config<Prec>(P, units_in, ws_n, force_plain, sig_f64, ws_budget(), c));
     // the two kernels keep different between-unit invariants: never share a workspace
-    Workspace& W = c.fr ? g.wsw : g.wsb;
+    Workspace& W = P.sched == FBC_SCHED_BATCHED && !force_plain && !sig_f64 ? g.wsw : g.wsb;
+    BlockCfg c;
+    FBC_TRY(block_config<Prec>(P, units_in, ws_n, force_plain, sig_f64, ws_budget(&W), c));
     FBC_TRY(ensure_ws(W, c.slots, c.stride, ws_n * c.K, (int)sizeof(typename Prec::D)));
     FBC_CK(g.units_b.ensure(sizeof(Unit) * c.units.size()));
     FBC_CK(cudaMemcpyAsync(g.units_b.p, c.units.data(), sizeof(Unit) * c.units.size(),
@@ -1097,12 +1123,9 @@ int launch_log(const Plan& P, std::vector<Unit>&& units, fbc_stats* st, int& lau
     int ws_n = 0;
     for (const Unit& u : units) ws_n = std::max(ws_n, P.segs[u.seg].n);
     LogCfg c;
-    FBC_TRY(log_config<Prec>(P, std::move(units), ws_n, ws_budget(), c));
     Workspace& W = g.wsl;
-    if (!W.buf.p || (int64_t)W.buf.cap < c.blocks * c.teams * c.stride) {
-        W.buf.release();
-        FBC_CK(W.buf.ensure((size_t)(c.blocks * c.teams * c.stride)));
-    }
+    FBC_TRY(log_config<Prec>(P, std::move(units), ws_n, ws_budget(&W), c));
+    FBC_CK(ws_take(W, c.blocks * c.teams * c.stride, false));
     FBC_CK(g.lunits.ensure(sizeof(Unit) * c.units.size()));
     FBC_CK(cudaMemcpyAsync(g.lunits.p, c.units.data(), sizeof(Unit) * c.units.size(), cudaMemcpyHostToDevice, g.st));
     if (st) st->h2d_bytes += (int64_t)(sizeof(Unit) * c.units.size());
@@ -2845,7 +2868,7 @@ int plan_capture(fbc_plan_s* p, Plan& P) {
     BlockCfg bc;
     KParams K = base;
     if (!ub.empty()) {
-        FBC_TRY(block_config<Prec>(P, ub, nb_max, false, false, ws_budget(), bc));
+        FBC_TRY(block_config<Prec>(P, ub, nb_max, false, false, ws_budget(nullptr), bc));
         if (!bc.fr) return FBC_OK;
         FBC_CK(p->bunits.ensure(sizeof(Unit) * bc.units.size()));
         FBC_CK(cudaMemcpyAsync(p->bunits.p, bc.units.data(), sizeof(Unit) * bc.units.size(), cudaMemcpyHostToDevice,
@@ -2877,7 +2900,8 @@ int plan_capture(fbc_plan_s* p, Plan& P) {
         int quad_launches = 0, nl_max = 0;
         for (const Unit& u : ul) nl_max = std::max(nl_max, P.segs[u.seg].n);
         FBC_TRY(log_quads_build(lb, p->segs.as<Seg>(), p->lsegs, p->lextra, quad_launches));
-        FBC_TRY(log_config<Prec>(P, std::move(ul), nl_max, ws_budget(), lc));
+        const int64_t budget = ws_budget(nullptr) - (ws_limit() > 0 ? (int64_t)p->ws.cap : 0);
+        FBC_TRY(log_config<Prec>(P, std::move(ul), nl_max, budget, lc));
         FBC_CK(p->lunits.ensure(sizeof(Unit) * lc.units.size()));
         FBC_CK(cudaMemcpyAsync(p->lunits.p, lc.units.data(), sizeof(Unit) * lc.units.size(), cudaMemcpyHostToDevice, g.st));
         FBC_CK(p->lws.ensure((size_t)(lc.blocks * lc.teams * lc.stride)));

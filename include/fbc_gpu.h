@@ -114,7 +114,8 @@ const char* fbc_last_error_string(void);
  *   "iter_mult"        distance-pass rounds are capped at iter_mult * (n + 2); 0 makes every unit
  *                      stop at once with FBC_ERR_ITER_LIMIT (a host-side way to exercise the
  *                      bounded-loop error path)
- *   "ws_budget_mb"     cap of the block kernels' workspace (0 = 60% of the free device memory)
+ *   "ws_budget_mb"     cap of the block kernels' kept workspaces together, and of a plan's own (0 = a launch
+ *                      may take 60% of the device memory that is free or its kernel's already)
  *   "debug_sched"      schedule of fbc_sssp_debug (0 plain, else batched)
  *   "scratch_keep_mb"  per-call scratch (graph builds, text parsing, class grouping) comes from a
  *                      stream-ordered memory pool that keeps up to this many MiB (default 8192)
