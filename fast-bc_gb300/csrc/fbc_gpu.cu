@@ -2433,8 +2433,12 @@ int fbc_single_source(fbc_graph G, int32_t source, int precision, double* out_de
     P.bc_len = G->n;
     P.sched = team_takes_blocks() && (team_fits(P, 0, 1) || log_fits(P, 0)) ? FBC_SCHED_BATCHED : FBC_SCHED_PLAIN;
     P.results.emplace_back(out_dep, sizeof(double) * (size_t)G->n);
-    FBC_TRY(run_plan(P, st));
-    FBC_TRY(download_bc(out_dep, G->n, false, st));
+    int rc = run_plan(P, st);
+    if (!rc) rc = download_bc(out_dep, G->n, false, st);
+    if (rc) {  // a failed call leaves zeros
+        std::fill(out_dep, out_dep + G->n, 0.0);
+        return rc;
+    }
     if (st) st->wall_ms = now_ms() - t0;
     return FBC_OK;
 }
