@@ -1390,14 +1390,20 @@ int check_sched(int sched) {
 }
 
 constexpr size_t kStageMax = (size_t)64 << 20;
-int ensure_stage(size_t bytes) {
-    if (g.stage && g.stage_cap >= bytes) return FBC_OK;
+// The kept page-locked memory, of at least that size; null where there is none to be had.
+void* ensure_stage(size_t bytes) {
+    if (g.stage && g.stage_cap >= bytes) return g.stage;
     if (g.stage) cudaFreeHost(g.stage);
     g.stage = nullptr;
     g.stage_cap = 0;
-    FBC_CK(cudaMallocHost(&g.stage, std::max<size_t>(bytes, 1 << 20)));
-    g.stage_cap = std::max<size_t>(bytes, 1 << 20);
-    return FBC_OK;
+    const size_t want = std::max<size_t>(bytes, 1 << 20);
+    if (cudaMallocHost(&g.stage, want) != cudaSuccess) {
+        (void)cudaGetLastError();
+        g.stage = nullptr;
+        return nullptr;
+    }
+    g.stage_cap = want;
+    return g.stage;
 }
 
 int download_bc(double* out, int64_t len, bool accumulate, fbc_stats* st) {
@@ -1405,12 +1411,13 @@ int download_bc(double* out, int64_t len, bool accumulate, fbc_stats* st) {
     // what is added to the caller's array comes through page-locked memory (kept, up to kStageMax bytes)
     std::vector<double> tmp;
     double* dst = out;
-    if (accumulate && sizeof(double) * (size_t)len <= kStageMax) {
-        FBC_TRY(ensure_stage(sizeof(double) * (size_t)len));
-        dst = (double*)g.stage;
-    } else if (accumulate) {
-        tmp.resize((size_t)len);
-        dst = tmp.data();
+    if (accumulate) {
+        const size_t bytes = sizeof(double) * (size_t)len;
+        dst = bytes <= kStageMax ? (double*)ensure_stage(bytes) : nullptr;
+        if (!dst) {
+            tmp.resize((size_t)len);
+            dst = tmp.data();
+        }
     }
     FBC_CK(cudaMemcpyAsync(dst, g.bc.p, sizeof(double) * (size_t)len, cudaMemcpyDeviceToHost, g.st));
     FBC_CK(cudaStreamSynchronize(g.st));
@@ -2277,20 +2284,21 @@ int fbc_graph_download(fbc_graph G, int64_t* row_ptr, int32_t* col, double* w) {
     if (!G->host_ok && G->m > 0) {  // built on the device: converted there, copied into the caller's arrays
         const size_t n1 = (size_t)G->n + 1, m = (size_t)G->m;
         TmpBuf drp, dcol, dw;
-        FBC_CK(drp.ensure(sizeof(int64_t) * n1));
-        FBC_CK(dcol.ensure(sizeof(int32_t) * m));
-        FBC_CK(dw.ensure(sizeof(double) * m));
-        fbc::gb_export_kernel<<<grid_for(G->m), 256, 0, g.st>>>(G->n, G->m, G->d_rp, G->d_adj, drp.as<int64_t>(),
-                                                                dcol.as<int32_t>(), dw.as<double>());
-        FBC_CK(cudaGetLastError());
-        if (row_ptr) fbc_host::prefault(row_ptr, sizeof(int64_t) * n1);
-        if (col) fbc_host::prefault(col, sizeof(int32_t) * m);
-        if (w) fbc_host::prefault(w, sizeof(double) * m);
-        if (row_ptr) FBC_CK(cudaMemcpyAsync(row_ptr, drp.p, sizeof(int64_t) * n1, cudaMemcpyDeviceToHost, g.st));
-        if (col) FBC_CK(cudaMemcpyAsync(col, dcol.p, sizeof(int32_t) * m, cudaMemcpyDeviceToHost, g.st));
-        if (w) FBC_CK(cudaMemcpyAsync(w, dw.p, sizeof(double) * m, cudaMemcpyDeviceToHost, g.st));
-        FBC_CK(cudaStreamSynchronize(g.st));
-        return FBC_OK;
+        if ((!row_ptr || drp.ensure(sizeof(int64_t) * n1) == cudaSuccess) &&
+            (!col || dcol.ensure(sizeof(int32_t) * m) == cudaSuccess) && (!w || dw.ensure(sizeof(double) * m) == cudaSuccess)) {
+            fbc::gb_export_kernel<<<grid_for(G->m), 256, 0, g.st>>>(G->n, G->m, G->d_rp, G->d_adj, drp.as<int64_t>(),
+                                                                    dcol.as<int32_t>(), dw.as<double>());
+            FBC_CK(cudaGetLastError());
+            if (row_ptr) fbc_host::prefault(row_ptr, sizeof(int64_t) * n1);
+            if (col) fbc_host::prefault(col, sizeof(int32_t) * m);
+            if (w) fbc_host::prefault(w, sizeof(double) * m);
+            if (row_ptr) FBC_CK(cudaMemcpyAsync(row_ptr, drp.p, sizeof(int64_t) * n1, cudaMemcpyDeviceToHost, g.st));
+            if (col) FBC_CK(cudaMemcpyAsync(col, dcol.p, sizeof(int32_t) * m, cudaMemcpyDeviceToHost, g.st));
+            if (w) FBC_CK(cudaMemcpyAsync(w, dw.p, sizeof(double) * m, cudaMemcpyDeviceToHost, g.st));
+            FBC_CK(cudaStreamSynchronize(g.st));
+            return FBC_OK;
+        }
+        (void)cudaGetLastError();  // no device memory for that: the host converts
     }
     FBC_TRY(ensure_host_csr(G));
     if (row_ptr) std::copy(G->h_rp.begin(), G->h_rp.end(), row_ptr);

@@ -110,15 +110,17 @@ __global__ void gb_merge_kernel(int32_t n, const int32_t* __restrict__ rs, const
     }
 }
 
-// The CSR in the caller's types: 64-bit offsets, destinations, weights as doubles.
+// The CSR in the caller's types: 64-bit offsets, destinations, weights as doubles (each null: not wanted).
 __global__ void gb_export_kernel(int32_t n, int64_t m, const int32_t* __restrict__ rp, const int2* __restrict__ adj,
                                  int64_t* __restrict__ rp64, int32_t* __restrict__ col, double* __restrict__ w) {
     const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t v = t0; v <= n; v += nt) rp64[v] = rp[v];
+    if (rp64)
+        for (int64_t v = t0; v <= n; v += nt) rp64[v] = rp[v];
+    if (!col && !w) return;
     for (int64_t e = t0; e < m; e += nt) {
         const int2 a = adj[e];
-        col[e] = a.x;
-        w[e] = (double)a.y;
+        if (col) col[e] = a.x;
+        if (w) w[e] = (double)a.y;
     }
 }
 
