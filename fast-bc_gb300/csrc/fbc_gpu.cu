@@ -1240,6 +1240,25 @@ int launch_old_blocks(const Plan& P, const OldSplit& o, fbc_stats* st, int& laun
     return launch_block<Prec>(P, small_first ? us_large : us_small, small_first ? nl_max : ns_max, st, launches);
 }
 
+// Units that were handed back, in the order of their segments and sources instead of that of their ends:
+// neighbouring sources share the rounds, levels and rows of a frontier block (5,000 sources of a path of 5,000
+// vertices 57 -> 48 ms, of a grid of 3 x 1,667 36.4 -> 32.3).
+void in_source_order(const Plan& P, std::vector<fbc::RetryRec>& rec) {
+    std::vector<int64_t> at(P.segs.size() + 1, 0);
+    for (size_t s = 0; s < P.segs.size(); ++s) at[s + 1] = at[s] + P.segs[s].n;
+    const auto key = [&](const fbc::RetryRec& r) { return at[r.u.seg] + r.u.src; };
+    if (at.back() > 8 * (int64_t)rec.size()) {
+        std::stable_sort(rec.begin(), rec.end(), [&](const fbc::RetryRec& a, const fbc::RetryRec& b) { return key(a) < key(b); });
+        return;
+    }
+    std::vector<int32_t> first((size_t)at.back() + 1, 0);
+    for (const auto& r : rec) ++first[(size_t)key(r) + 1];
+    for (size_t k = 1; k < first.size(); ++k) first[k] += first[k - 1];
+    std::vector<fbc::RetryRec> out(rec.size());
+    for (const auto& r : rec) out[(size_t)first[(size_t)key(r)]++] = r;
+    rec.swap(out);
+}
+
 // Upload the plan, launch, wait, and check the device status.  Results stay on the device
 // (g.bc, g.bdist, g.bsig) for the caller to download.
 template <class Prec>
@@ -1327,6 +1346,7 @@ int run_plan_t(Plan& P, fbc_stats* st) {
         std::vector<fbc::RetryRec> rec((size_t)err[1]);
         if (st) st->retries += err[1];
         FBC_CK(cudaMemcpy(rec.data(), g.retry.p, sizeof(fbc::RetryRec) * rec.size(), cudaMemcpyDeviceToHost));
+        in_source_order(P, rec);
         std::vector<Unit> to64, tof64, narrow;
         int nmax = 0;
         for (const auto& r : rec) {
