@@ -178,6 +178,7 @@ struct fbc_graph_s {
     int32_t maxw = 0;
     int32_t maxindeg = 0;
     int32_t maxdeg = 0;  // longest row
+    double ties = 0.0;   // share of the vertices within two edges that have several shortest ways (gb_ties_kernel)
     double meanw = 1.0;
     int32_t* d_rp = nullptr;
     int2* d_adj = nullptr;
@@ -256,6 +257,21 @@ int check_init(DevGuard& dg) {
     return FBC_OK;
 }
 
+// The graph's ties, from a sample of its uploaded rows (waits for the stream).
+cudaError_t graph_ties(fbc_graph_s* G) {
+    cudaError_t e = g.ctr.ensure(64);
+    if (e == cudaSuccess) e = cudaMemsetAsync(g.ctr.p, 0, 64, g.st);
+    if (e != cudaSuccess) return e;
+    int* const d = g.ctr.as<int>();
+    int t[2] = {0, 0};  // vertices within two edges of the sample, tied ones
+    fbc::gb_ties_kernel<<<fbc::kTieSamples / fbc::kTieWarps, 32 * fbc::kTieWarps, 0, g.st>>>(G->n, G->d_rp, G->d_adj, d, d + 1);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(t, d, sizeof(t), cudaMemcpyDeviceToHost, g.st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(g.st);
+    G->ties = t[0] > 0 ? (double)t[1] / (double)t[0] : 0.0;
+    return e;
+}
+
 // Validate a host CSR with double weights and build the device graph.
 int make_graph(int32_t n, std::vector<int64_t>&& rp, std::vector<int32_t>&& col, const double* w,
                fbc_graph* out) {
@@ -313,8 +329,9 @@ int make_graph(int32_t n, std::vector<int64_t>&& rp, std::vector<int32_t>&& col,
                                      cudaMemcpyHostToDevice, g.st);
     cudaError_t e4 = cudaMemcpyAsync(G->d_adj, adj.data(), sizeof(int2) * adj.size(),
                                      cudaMemcpyHostToDevice, g.st);
-    cudaError_t e5 = cudaStreamSynchronize(g.st);
+    cudaError_t e5 = graph_ties(G);
     if (e3 != cudaSuccess || e4 != cudaSuccess || e5 != cudaSuccess) {
+        cudaStreamSynchronize(g.st);
         cudaFree(G->d_rp);
         cudaFree(G->d_adj);
         delete G;
@@ -339,6 +356,7 @@ struct Plan {
     std::vector<int32_t> seg_maxw;
     std::vector<int32_t> seg_maxindeg;
     std::vector<int32_t> seg_maxdeg;
+    std::vector<double> seg_ties;
     std::vector<std::pair<void*, size_t>> results;  // host memory that the call fills after the launches
     std::vector<uint4**> seg_quads;  // where a whole graph keeps its quads (null: a community)
     std::vector<Unit> units;
@@ -831,6 +849,22 @@ bool team_fits(const Plan& P, size_t s, int64_t units) {
            n + P.seg_m[s] / 3 + 1 <= 65535 && (units <= 4 * (int64_t)g.nsm ? 1 : 2) * fbc::team_bytes(n, P.seg_maxdeg[s] > 8) <= team_dyn_smem();
 }
 
+// Segments whose path counts will outgrow 24 bits on most sources, by the share of ties within two edges and
+// the hops across the segment, about the root of its vertices over their edges: counts grow with the ties on the
+// way.  Such units would be run, given back and done again, so they start with the kernels of wider counts.  Share
+// squared x vertices / edges a vertex, and what came back (all sources, 2,432 of geometric graphs above 10,000
+// vertices): geometric graphs (3-NN) of 8,192 vertices 3.0: none, 16,000 7.7: half; 6-NN of 8,000 5.9: 11%; grids
+// of one weight 14 x 14 5.6: none, 16 x 16 7.3: 16%, 18 x 18 9.2: 40%, 30 x 30 25: all; of two weights 30 x 30
+// 3.5: none, 90 x 71 23: all; of weights to 8 90 x 71 1.4: none.  Device time with the units begun here and in the
+// older kernels at once: 6-NN 25.1 against 49.6 ms; geometric 16,000 16.6 / 15.7; 18 x 18 0.82 / 0.74; 30 x 30
+// 1.03 / 0.91; 8 x 500 10.1 / 9.2; 4 x 500 8.2 / 6.4.  Below the least share, ties are too few to multiply (road
+// weights of 1 to 100 on four million vertices: 0.0025, 6.6, none).
+constexpr double kTieShare = 0.02, kTieMost = 7.0;
+bool tie_rich(const Plan& P, size_t s) {
+    const double t = P.seg_ties[s], n = P.segs[s].n;
+    return t >= kTieShare && t * t * n * n >= kTieMost * (double)P.seg_m[s];
+}
+
 // Segments above warp_max_n go to the team kernel too, unless an option asks for the frontier
 // kernel: warp_max_n = 0 (no segment in shared memory) or a forced number of sources per block.
 bool team_takes_blocks() { return g.opt.warp_max_n > 0 && g.opt.group == 0; }
@@ -1279,7 +1313,7 @@ int run_plan_t(Plan& P, fbc_stats* st) {
     // warp_max_n in one launch (with what the one-warp kernel takes, the first timed phase) and
     // above it in another; the rest run block-per-source.
     std::vector<Unit> rest, tw, tb, lg;
-    std::vector<char> team(P.segs.size(), 0), logs(P.segs.size(), 0);
+    std::vector<char> team(P.segs.size(), 0), logs(P.segs.size(), 0), ties(P.segs.size(), 0);
     if (P.sched == FBC_SCHED_BATCHED && !P.dbg_dist) {  // debug dumps come from block kernels
         const bool blocks = team_takes_blocks();
         for (size_t s = 0; s < P.segs.size(); ++s)
@@ -1287,8 +1321,12 @@ int run_plan_t(Plan& P, fbc_stats* st) {
             const bool up_to = P.segs[s].n <= std::min<int64_t>(g.opt.warp_max_n, 65535);
             team[s] = (up_to || blocks) && team_fits(P, s, (int64_t)P.units.size());
             logs[s] = !team[s] && !up_to && blocks && log_fits(P, s);
+            ties[s] = (team[s] || logs[s]) && tie_rich(P, s);
+            if (ties[s]) team[s] = logs[s] = 0;
         }
     }
+    if (st)
+        for (const Unit& u : P.units) st->retries += ties[u.seg];
     int64_t nwarp = 0, nblock = 0;  // units of the two phases
     double warp_bytes = 0, block_bytes = 0;
     for (const Unit& u : P.units) {
@@ -1670,6 +1708,7 @@ int prepare_clusters(const fbc_graph_s* G, int32_t nclusters, const int64_t* cof
         P.seg_maxw.push_back(G->maxw);
         P.seg_maxindeg.push_back(G->maxindeg);
         P.seg_maxdeg.push_back(G->maxdeg);
+        P.seg_ties.push_back(G->ties);
         for (int32_t i = 0; i < s.n; ++i) P.units.push_back(Unit{c, i, 1.0, ent + (int64_t)i * s.nb});
         ent += (int64_t)s.n * s.nb;
     }
@@ -1721,8 +1760,8 @@ int device_csr_build(int64_t count, const int32_t* dsrc, const int32_t* ddst, co
     TmpBuf ints, deg, rs, cursor, keys, ndeg, indeg;
     FBC_CK(ints.ensure(64));
     // ints: [0] max source, [1] error bits, [2] max weight, [3] max in-degree, [4..5] weight sum,
-    // [6] longest row
-    int hi[7] = {-1, 0, 0, 0, 0, 0, 0};
+    // [6] longest row, [8] vertices within two edges of a sample, [9] tied ones
+    int hi[10] = {-1, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     FBC_CK(cudaMemcpyAsync(ints.p, hi, sizeof(hi), cudaMemcpyHostToDevice, g.st));
     int* di = ints.as<int>();
     fbc::gb_check_kernel<<<grid_for(count), 256, 0, g.st>>>(count, dsrc, ddst,
@@ -1786,6 +1825,7 @@ int device_csr_build(int64_t count, const int32_t* dsrc, const int32_t* ddst, co
                                                         dw, G->d_rp, G->d_adj, indeg.as<int32_t>(),
                                                         di + 2, (unsigned long long*)(di + 4), di + 6, di + 1);
     fbc::gb_max_kernel<<<grid_for(n), 256, 0, g.st>>>(n, indeg.as<int32_t>(), di + 3);
+    fbc::gb_ties_kernel<<<fbc::kTieSamples / fbc::kTieWarps, 32 * fbc::kTieWarps, 0, g.st>>>(n, G->d_rp, G->d_adj, di + 8, di + 9);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(hi, ints.p, sizeof(hi), cudaMemcpyDeviceToHost, g.st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(g.st);
@@ -1797,6 +1837,7 @@ int device_csr_build(int64_t count, const int32_t* dsrc, const int32_t* ddst, co
     G->maxw = hi[2];
     G->maxindeg = hi[3];
     G->maxdeg = hi[6];
+    G->ties = hi[8] > 0 ? (double)hi[9] / (double)hi[8] : 0.0;
     G->meanw = medges ? (double)sumw / (double)medges : 1.0;
     if ((double)n * (double)G->maxw > 2147483646.0) {
         drop();
@@ -2386,6 +2427,7 @@ int fbc_exact_bc(fbc_graph G, int precision, int sched, double* out_bc, fbc_stat
     P.seg_maxw.push_back(G->maxw);
     P.seg_maxindeg.push_back(G->maxindeg);
     P.seg_maxdeg.push_back(G->maxdeg);
+    P.seg_ties.push_back(G->ties);
     for (int32_t s = 0; s < G->n; ++s) P.units.push_back(Unit{0, s, 1.0, -1});
     P.bc_len = G->n;
     P.results.emplace_back(out_bc, sizeof(double) * (size_t)G->n);
@@ -2420,6 +2462,7 @@ int fbc_sssp_dependency_batch(fbc_graph G, int64_t count, const int32_t* sources
     P.seg_maxw.push_back(G->maxw);
     P.seg_maxindeg.push_back(G->maxindeg);
     P.seg_maxdeg.push_back(G->maxdeg);
+    P.seg_ties.push_back(G->ties);
     for (int64_t i = 0; i < count; ++i)
         P.units.push_back(Unit{0, map ? map[sources[i]] : sources[i], cards ? cards[i] : 1.0, -1});
     // on a relabelled graph, sources in the locality order: the sources running at once then
@@ -2457,9 +2500,10 @@ int fbc_single_source(fbc_graph G, int32_t source, int precision, double* out_de
     P.seg_maxw.push_back(G->maxw);
     P.seg_maxindeg.push_back(G->maxindeg);
     P.seg_maxdeg.push_back(G->maxdeg);
+    P.seg_ties.push_back(G->ties);
     P.units.push_back(Unit{0, source, 1.0, -1});
     P.bc_len = G->n;
-    P.sched = team_takes_blocks() && (team_fits(P, 0, 1) || log_fits(P, 0)) ? FBC_SCHED_BATCHED : FBC_SCHED_PLAIN;
+    P.sched = team_takes_blocks() && (team_fits(P, 0, 1) || log_fits(P, 0)) && !tie_rich(P, 0) ? FBC_SCHED_BATCHED : FBC_SCHED_PLAIN;
     P.results.emplace_back(out_dep, sizeof(double) * (size_t)G->n);
     int rc = run_plan(P, st);
     if (!rc) rc = download_bc(out_dep, G->n, false, st);
@@ -3142,6 +3186,7 @@ int fbc_multi_exact_bc(int32_t ngraphs, const fbc_graph* graphs, int precision, 
         P.seg_maxw.push_back(graphs[i]->maxw);
         P.seg_maxindeg.push_back(graphs[i]->maxindeg);
         P.seg_maxdeg.push_back(graphs[i]->maxdeg);
+        P.seg_ties.push_back(graphs[i]->ties);
         for (int32_t s = 0; s < graphs[i]->n; ++s) P.units.push_back(Unit{i, s, 1.0, -1});
         base[i + 1] = base[i] + graphs[i]->n;
     }
@@ -3173,6 +3218,7 @@ int fbc_sssp_debug(fbc_graph G, int32_t source, int32_t* out_dist, uint64_t* out
     P.seg_maxw.push_back(G->maxw);
     P.seg_maxindeg.push_back(G->maxindeg);
     P.seg_maxdeg.push_back(G->maxdeg);
+    P.seg_ties.push_back(G->ties);
     P.units.push_back(Unit{0, source, 1.0, -1});
     P.bc_len = G->n;
     P.dbg_sig = (unsigned long long*)base;

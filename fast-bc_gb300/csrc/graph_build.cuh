@@ -110,6 +110,63 @@ __global__ void gb_merge_kernel(int32_t n, const int32_t* __restrict__ rs, const
     }
 }
 
+// How rich a graph is in ties: of the vertices within two edges of a sample of vertices, how many are reached by
+// several shortest ones of these ways.  A warp per sampled vertex; of longer rows the first kTieRow edges.
+constexpr int kTieRow = 16;
+constexpr int kTieSamples = 1024;
+constexpr int kTieWarps = 4;  // of a block
+__global__ void __launch_bounds__(32 * kTieWarps) gb_ties_kernel(int32_t n, const int32_t* __restrict__ rp,
+                                                                 const int2* __restrict__ adj, int* targets, int* tied) {
+    __shared__ uint2 ways[kTieWarps][kTieRow * (kTieRow + 1)];  // (vertex, length)
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    uint2* const way = ways[wid];
+    int nt = 0, nd = 0;
+    const int samples = min(n, kTieSamples);
+    for (int k = blockIdx.x * kTieWarps + wid; k < samples; k += gridDim.x * kTieWarps) {
+        const int u = (int)((int64_t)k * n / samples);
+        const int e = rp[u], deg = min(rp[u + 1] - e, kTieRow);
+        int2 a = make_int2(0, 0);
+        int f = 0, len = 0;
+        if (lane < deg) {
+            a = adj[e + lane];
+            f = rp[a.x];
+            len = min(rp[a.x + 1] - f, kTieRow);
+        }
+        int cnt = 0;
+        for (int i = 0; i < deg; ++i) {
+            const int x = __shfl_sync(0xffffffffu, a.x, i), w = __shfl_sync(0xffffffffu, a.y, i);
+            const int fi = __shfl_sync(0xffffffffu, f, i), li = __shfl_sync(0xffffffffu, len, i);
+            if (lane == li) way[cnt + li] = make_uint2((unsigned)x, (unsigned)w);
+            if (lane < li) {
+                const int2 b = adj[fi + lane];
+                way[cnt + lane] = make_uint2((unsigned)b.x, (unsigned)w + (unsigned)b.y);
+            }
+            cnt += li + 1;
+        }
+        __syncwarp();
+        for (int r = lane; r < cnt; r += 32) {
+            const uint2 me = way[r];
+            int same = 0;
+            bool least = me.x != (unsigned)u;  // the first of the shortest ways to this vertex
+            for (int q = 0; q < cnt; ++q) {
+                const uint2 o = way[q];
+                if (o.x != me.x) continue;
+                if (o.y < me.y || (o.y == me.y && q < r)) least = false;
+                same += o.y == me.y;
+            }
+            nd += least;
+            nt += least && same > 1;
+        }
+        __syncwarp();
+    }
+    nt = __reduce_add_sync(0xffffffffu, nt);
+    nd = __reduce_add_sync(0xffffffffu, nd);
+    if (lane == 0 && nd) {
+        atomicAdd(targets, nd);
+        if (nt) atomicAdd(tied, nt);
+    }
+}
+
 // The CSR in the caller's types: 64-bit offsets, destinations, weights as doubles (each null: not wanted).
 __global__ void gb_export_kernel(int32_t n, int64_t m, const int32_t* __restrict__ rp, const int2* __restrict__ adj,
                                  int64_t* __restrict__ rp64, int32_t* __restrict__ col, double* __restrict__ w) {

@@ -72,8 +72,9 @@ typedef struct {
     int64_t warp_units;
     int64_t block_units;
     int32_t group;           /* sources per block of the log or the frontier kernel (0: neither launched) */
-    int32_t retries;         /* units recomputed by another kernel: path counts too wide for the first one,
-                                or more rounds than it keeps */
+    int32_t retries;         /* units that another kernel did than their size calls for: path counts too wide for
+                                that one (found out there, or foreseen from the graph's ties and then not begun
+                                there), or more rounds than it keeps */
 } fbc_stats;
 
 /* Library lifetime.  fbc_gpu_init selects the device and creates the library stream. */
