@@ -100,7 +100,7 @@ struct KParams {
     RetryRec* retry;
     int32_t retry_cap;
     int2* gave;                  // team and log kernels, per segment: units ended, units of these given
-                                 // back for wider counts (null: not counted)
+                                 // back or better done elsewhere (null: not counted)
     int32_t cnt_bits;            // frontier kernel: counter / mask bits next to the path count
     int32_t* dbg_dist;           // debug dump of one unit (may be null)
     unsigned long long* dbg_sig;
@@ -118,13 +118,21 @@ __device__ __forceinline__ void request_retry(const KParams& P, const Unit& u, i
     else atomicOr(P.err, kErrQueue);
 }
 
-// Units of a segment of which more than a third came back are handed back unstarted: a unit given back
+// More rounds than four times the root of n, when a source of the team and log kernels is looked at for narrow ones
+// (a road-like source has run two to three times the root by its end).
+__device__ __forceinline__ bool many_rounds(int n, int nr) { return (float)nr * (float)nr > 16.0f * (float)n; }
+
+// Units of a segment of which more than a third came back (or were too narrow) are handed back unstarted: a unit given back
 // has cost its distances and counts, about 0.6 of its time here, and is done again by a kernel that takes
 // a third longer, so with more than that it is better begun there.
 __device__ __forceinline__ bool gave_up(const KParams& P, int seg) {
     if (!P.gave) return false;
     const int2 c = __ldcg(P.gave + seg);
     return c.x >= 16 && 3 * c.y > c.x;
+}
+// A source that was done, but is better done elsewhere: its segment's others, too.
+__device__ __forceinline__ void count_narrow(const KParams& P, int seg) {
+    if (P.gave) atomicAdd(&P.gave[seg].y, 1);
 }
 __device__ __forceinline__ void count_unit(const KParams& P, int seg, bool back) {
     if (!P.gave) return;

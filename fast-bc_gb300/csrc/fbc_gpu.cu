@@ -1274,6 +1274,13 @@ int launch_old_blocks(const Plan& P, const OldSplit& o, fbc_stats* st, int& laun
     return launch_block<Prec>(P, small_first ? us_large : us_small, small_first ? nl_max : ns_max, st, launches);
 }
 
+// Many units that the team kernel hands back run in the plain kernel (64-bit counts) up to this size, where its
+// small blocks are faster than the one-warp kernel; few, and larger ones, in the one-warp or frontier kernel.  All
+// sources of a path, plain / one-warp or frontier kernel, ms: 1,500 vertices 6.6 / 8.2, 3,000 22.3 / 44.4, 4,000 33.2 /
+// 32.9, 5,000 52 / 45; 3 x 800 5.8 / 9.9; of a grid of one weight 50 x 50 2.4 / 5.3.  One source of a path of 1,500:
+// 4.2 with the team kernel's part, 1.7 through the one-warp kernel.
+constexpr int kPlainBack = 4096;
+
 // Units that were handed back, in the order of their segments and sources instead of that of their ends:
 // neighbouring sources share the rounds, levels and rows of a frontier block (5,000 sources of a path of 5,000
 // vertices 57 -> 48 ms, of a grid of 3 x 1,667 36.4 -> 32.3).
@@ -1388,8 +1395,10 @@ int run_plan_t(Plan& P, fbc_stats* st) {
         std::vector<Unit> to64, tof64, narrow;
         int nmax = 0;
         for (const auto& r : rec) {
-            (r.code == fbc::kErrNarrow ? narrow : r.code == fbc::kErrRetry ? to64 : tof64).push_back(r.u);
-            nmax = std::max(nmax, P.segs[r.u.seg].n);
+            const int n = P.segs[r.u.seg].n;
+            const bool wider = r.code == fbc::kErrNarrow && (n > kPlainBack || rec.size() <= 8 * (size_t)g.nsm);
+            (wider ? narrow : r.code != fbc::kErrSigma ? to64 : tof64).push_back(r.u);
+            if (!wider) nmax = std::max(nmax, n);
         }
         if (!narrow.empty()) {  // counts above the team kernel's 32 bits: the kernels with wider ones
             OldSplit ns;

@@ -156,6 +156,16 @@ __device__ __forceinline__ T lload(const T* p) {
     else return *p;
 }
 
+// Narrow sources: those of more rounds to come than are kept stop early, and so do, where there are several waves
+// of units on a segment whose sources the frontier kernel's blocks share by four, those of less than twenty pops a
+// round; with less than 27 the segment's other units start there.  All sources, this kernel / that one, ms: 6 x
+// 2,000 vertices 125 / 92, 12 x 1,500 164 / 136, 20 x 1,000 138 / 121, 32 x 600 90 / 86, 40 x 500 82 / 82, 64 x 300
+// 60 / 68 (a square's corner has some fifty pops a round).
+template <int kThreads>
+__device__ __forceinline__ bool log_shared(const KParams& P, int n) {
+    return P.gave && n <= 32768 && P.nunits > 4 * ((int64_t)gridDim.x * (blockDim.x / kThreads));
+}
+
 // One source by a team of kThreads threads (bar: its named barrier), or by the `threads` threads of a
 // cluster of blocks, whose control words lie in the first block's shared memory.  tid numbers the team's
 // threads, whole warps together.
@@ -282,6 +292,7 @@ __device__ __forceinline__ void log_unit(const KParams& P, const Seg& sg, const 
                 nfar += *(volatile int*)&C.far[cs];
             } else {
                 if (nfar == 0) break;
+                if (many_rounds(n, nr) && e < (log_shared<kThreads>(P, n) ? 20 : 3) * nr) { bad = kErrNarrow; break; }
                 // the threshold moves on to the bucket of the closest live far vertex
                 sync();  // (C.dmin is set)
                 const uint32_t* const qo = fs ? S.far1 : S.far0;
@@ -329,6 +340,7 @@ __device__ __forceinline__ void log_unit(const KParams& P, const Seg& sg, const 
         delta = max(1, delta >> 2);
         sync();
     }
+    if (tid == 0 && !bad && many_rounds(n, 2 * nr) && total < 27 * nr && log_shared<kThreads>(P, n)) count_narrow(P, u.seg);
 
     if (!bad) {
         // --------------------------------------------------------------- path counts, in pop order

@@ -12,9 +12,10 @@
 //     (1% more pops on road grids; the log's rounds outnumber the DAG's levels by a fifth);
 //   * 13.5 bytes of state per vertex, planes reused pass after pass:
 //       plane 0   (dist | stamp) word                    -> low word of the coefficient
-//       plane 1   log of the pops (16 bits, two per vertex; a pop that a later one replaces is cleared)
+//       plane 1   log of the pops (16 bits, two per vertex; a pop that a later one replaces is cleared), and from
+//                 its far end the rounds' first log places
 //       plane 2   log place of the last pop              -> path count (32 bits) -> high word
-//     an 8-bit tight-edge mask (16 bits for rows of 9 to 16 edges) and the rounds' first log places.
+//     an 8-bit tight-edge mask (16 bits for rows of 9 to 16 edges).
 //     Path counts stay below 2^24 here; a source that needs more, or more rounds than are kept, stops
 //     before its dependencies and is done by the kernels with wider counts;
 //   * no far pile: when a bucket is empty, the next bucket's vertices are found by a sweep over the words
@@ -74,10 +75,11 @@ struct TeamParams {
 };
 
 __host__ __device__ inline int64_t team_n16(int64_t n) { return (n + 15) & ~int64_t(15); }
-// shared-memory state of one source
-__host__ __device__ inline int64_t team_rounds(int64_t n16) { return n16 / 4 + 64; }  // kept rounds
+// shared-memory state of one source: beside the log room for n / 4 rounds; more (narrow sources) lie in its end
+__host__ __device__ inline int team_round_bytes(int64_t n16) { return (int)al16(n16 / 2 + 130); }
+__host__ __device__ inline int64_t team_rounds(int64_t n16) { return n16 / 2 + 256; }  // kept rounds
 __host__ __device__ inline int64_t team_bytes(int64_t n, bool wide_mask) {
-    return (wide_mask ? 14 : 13) * team_n16(n) + al16(2 * team_rounds(team_n16(n)) + 2);
+    return (wide_mask ? 14 : 13) * team_n16(n) + team_round_bytes(team_n16(n));
 }
 
 // Quads of the team segments, one grid row of blocks per segment: the rows in their order, a row
@@ -254,6 +256,18 @@ struct CoefBits<float2> {
     }
 };
 
+// Whether a source is too narrow for the kernel after nr rounds of e pops together: more rounds to come than are
+// kept; and, where there are several waves of units (so that most of the segment's are then not begun), rounds that
+// the block's few sources cannot fill.  All sources, this kernel against those of the frontier kernel, ms: 10 x 700
+// vertices (two at once on an SM, 12 to 22 pops a round) 36.2 / 26.9, 5 x 1,000 (three; 6 to 11) 33.7 / 21.6; but
+// 16 x 350 (16 to 28) 11.2 / 12.8, 12 x 340 6.5 / 9.4, 8 x 500 (four; 9 to 15) 9.0 / 11.3.
+constexpr int kTeamMany = 16;  // units a block
+__device__ __forceinline__ bool team_narrow(const KParams& K, int n, int nr, int e) {
+    const float left = (float)n * (float)nr / (float)e;  // rounds that n pops take at this pace
+    return left > 0.9f * (float)team_rounds(team_n16(n)) ||
+           (K.gave && K.nunits > kTeamMany * (int64_t)gridDim.x && (float)n * left > 2e6f);
+}
+
 template <class Prec, bool kWarp, bool kRows>
 __device__ __forceinline__ void TeamUnit<Prec, kWarp, kRows>::run(const KParams& K, const Seg& sg, const Unit& u,
                                                                   const TeamSeg& ts, int off, int& delta) {
@@ -261,14 +275,16 @@ __device__ __forceinline__ void TeamUnit<Prec, kWarp, kRows>::run(const KParams&
     const int n16 = (int)team_n16(n);
     char* const base = team_smem + off;
     uint32_t* const word = (uint32_t*)base;                // plane 0
-    uint32_t* const sig = (uint32_t*)(base + 8 * n16);     // plane 2
+    const int rb = team_round_bytes(n16);
+    uint32_t* const sig = (uint32_t*)(base + 8 * n16 + rb);  // plane 2
     const bool wide = ts.wide_mask != 0;
-    // addresses: planes 0 and 2, the log (plane 1, 2 * n16 pops), where a vertex was popped last (plane
-    // 2 in the distance pass), tight-edge masks, round starts
-    const uint32_t aword = smem_addr(base), alog = aword + 4u * (uint32_t)n16, asig = aword + 8u * (uint32_t)n16,
-                   alast = asig, amask = aword + 12u * (uint32_t)n16, amask2 = amask + (uint32_t)n16,
-                   arnd = amask + (wide ? 2u : 1u) * (uint32_t)n16;
-    const int logcap = 2 * n16, rndcap = (int)team_rounds(n16);
+    // addresses: planes 0 and 2, the log (plane 1, 2 * n16 pops and what the rounds leave of theirs), the first
+    // round's start (the next ones' below it), where a vertex was popped last (plane 2 in the distance pass),
+    // tight-edge masks
+    const uint32_t aword = smem_addr(base), alog = aword + 4u * (uint32_t)n16,
+                   arnd = alog + 4u * (uint32_t)n16 + (uint32_t)rb - 2u, asig = arnd + 2u, alast = asig,
+                   amask = asig + 4u * (uint32_t)n16, amask2 = amask + (uint32_t)n16;
+    const int rndcap = (int)team_rounds(n16);
     const int sb = ts.stamp_bits;
     const uint32_t smask = (1u << sb) - 1u, one = 1u << sb;
     const int dinf = (int)(kNoEdge >> sb);                 // unreached: all distance bits set
@@ -319,7 +335,7 @@ __device__ __forceinline__ void TeamUnit<Prec, kWarp, kRows>::run(const KParams&
                 }
                 if (nr == rndcap) { bad = kErrNarrow; break; }
                 const uint32_t st = --stamp;
-                if (tid == 0) sts16(arnd + 2u * (uint32_t)nr, (uint32_t)s);
+                if (tid == 0) sts16(arnd - 2u * (uint32_t)nr, (uint32_t)s);
                 ++nr;
                 for (int b = s + (tid & ~31); b < e; b += nth) {
                     const int i = b + lane;
@@ -347,7 +363,7 @@ __device__ __forceinline__ void TeamUnit<Prec, kWarp, kRows>::run(const KParams&
                             const uint32_t old = atom_min_ge0(a, aword + x4[t], key);
                             want[t] = near && key < old && (old & smask) != st;
                         }
-                        push(want, x4, alog + 2u * (uint32_t)e, alog + 2u * (uint32_t)logcap, nn, cnt);
+                        push(want, x4, alog + 2u * (uint32_t)e, arnd - 2u * (uint32_t)nr, nn, cnt);
                         const bool link = quad_linked(q);
                         if (!__any_sync(kFull, link)) break;
                         const uint32_t next = link ? 4u * (q.w & 0xffffu) : v4;
@@ -356,6 +372,7 @@ __device__ __forceinline__ void TeamUnit<Prec, kWarp, kRows>::run(const KParams&
                     }
                 }
             } else {
+                if (many_rounds(n, nr) && team_narrow(K, n, nr, e)) { bad = kErrNarrow; break; }
                 // the bucket is empty: on to the next one, or to the one of the closest vertex beyond
                 const int T0 = T;
                 T = T0 >= dinf - delta ? dinf : T0 + delta;
@@ -371,7 +388,7 @@ __device__ __forceinline__ void TeamUnit<Prec, kWarp, kRows>::run(const KParams&
                         want[t] = d >= T0 && d < T;
                         if (d >= T) dmin = min(dmin, d);
                     }
-                    push(want, x4, alog + 2u * (uint32_t)e, alog + 2u * (uint32_t)logcap, nn, cnt);
+                    push(want, x4, alog + 2u * (uint32_t)e, arnd - 2u * (uint32_t)nr, nn, cnt);
                 }
                 dmin = __reduce_min_sync(kFull, dmin);
                 if constexpr (!kWarp) {
@@ -387,7 +404,7 @@ __device__ __forceinline__ void TeamUnit<Prec, kWarp, kRows>::run(const KParams&
             }
             s = e;
             e += nn;
-            if (e > logcap) { full = true; break; }
+            if (alog + 2u * (uint32_t)e > arnd - 2u * (uint32_t)nr) { full = true; break; }
         }
         sync();
         total = e;
@@ -395,6 +412,7 @@ __device__ __forceinline__ void TeamUnit<Prec, kWarp, kRows>::run(const KParams&
         // more than two pops a vertex: again with narrower buckets (width 1 pops every vertex once)
         delta = max(1, delta >> 2);
     }
+    if (tid == 0 && !bad && many_rounds(n, nr) && team_narrow(K, n, nr, total)) count_narrow(K, u.seg);
 
     if (!bad) {
         // --------------------------------------------------------------- path counts
@@ -405,15 +423,15 @@ __device__ __forceinline__ void TeamUnit<Prec, kWarp, kRows>::run(const KParams&
                 const int d = (int)(word[sg.border[j]] >> sb);
                 K.bdist[u.bout + j] = d != dinf ? nonneg_int_to_double(d) : 0.0;
             }
-        if (tid == 0) sts16(arnd + 2u * (uint32_t)nr, (uint32_t)total);
+        if (tid == 0) sts16(arnd - 2u * (uint32_t)nr, (uint32_t)total);
         fill(sig, n16 >> 2, 0u);
         sync();
         if (tid == 0) sts32(asig + src4, 1u);  // one path to the source
         sync();
         uint32_t high = 0u;  // bits of the counts
-        int s = 0, e = (int)lds16(arnd + 2u);
+        int s = 0, e = (int)lds16(arnd - 2u);
         for (int r = 0; r < nr; ++r) {
-            const int e2 = (int)lds16(arnd + 2u * (uint32_t)min(r + 2, nr));
+            const int e2 = (int)lds16(arnd - 2u * (uint32_t)min(r + 2, nr));
             for (int b = s + (tid & ~31); b < e; b += nth) {
                 const int i = b + lane;
                 uint32_t v4 = lds16(alog + 2u * (uint32_t)min(i, e - 1));
@@ -471,9 +489,9 @@ __device__ __forceinline__ void TeamUnit<Prec, kWarp, kRows>::run(const KParams&
         const double card = u.card;
         const bool card1 = __double_as_longlong(card) == 0x3ff0000000000000ll;
         double* const bc = K.bc + sg.out_base;
-        int hi = total, lo = (int)lds16(arnd + 2u * (uint32_t)(nr - 1));
+        int hi = total, lo = (int)lds16(arnd - 2u * (uint32_t)(nr - 1));
         for (int r = nr - 1; r >= 0; --r) {
-            const int lo2 = (int)lds16(arnd + 2u * (uint32_t)max(r - 1, 0));
+            const int lo2 = (int)lds16(arnd - 2u * (uint32_t)max(r - 1, 0));
             for (int b = lo + (tid & ~31); b < hi; b += nth) {
                 const int i = b + lane;
                 uint32_t v4 = lds16(alog + 2u * (uint32_t)min(i, hi - 1));
