@@ -52,6 +52,7 @@ int fail(int code, const std::string& msg) {
         cudaError_t e_ = (call);                                                         \
         if (e_ != cudaSuccess) {                                                         \
             int code_ = (e_ == cudaErrorMemoryAllocation) ? FBC_ERR_OOM : FBC_ERR_CUDA;  \
+            (void)cudaGetLastError(); /* not the next launch's */                        \
             return fail(code_, std::string(#call) + ": " + cudaGetErrorString(e_));      \
         }                                                                                \
     } while (0)
