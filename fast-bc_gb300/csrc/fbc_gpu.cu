@@ -226,17 +226,29 @@ struct fbc_plan_s {
     std::vector<int32_t> cverts, borders;
     Options opt;             // as they were when the plan was made: a capture after a run follows them too
     std::vector<char> wide;  // communities whose counts outgrew the team or log kernel in a run
-    // frees everything the plan holds, also when its creation stopped half way
-    ~fbc_plan_s() {
-        DevGuard dg_;
-        if (g.init) {  // no launch in flight still uses a buffer
-            dg_.enter();
-            cudaStreamSynchronize(g.st);
-        }
+    // Drops a capture, whole or begun, so that another can be made.  It may lay the slots out differently
+    // (other communities, other free memory), and the frontier kernel takes a slot whose header is not zero as one
+    // it has set up, so the new one starts from cleared slots.
+    void discard() {
+        if (g.init) cudaStreamSynchronize(g.st);  // no launch in flight still uses a buffer
         for (int i = 0; i < 2; ++i) {
             if (exec[i]) cudaGraphExecDestroy(exec[i]);
             if (graph[i]) cudaGraphDestroy(graph[i]);
+            exec[i] = nullptr;
+            graph[i] = nullptr;
         }
+        captured = false;
+        wbytes = bbytes = 0;
+        wunits = bunits_n = 0;
+        launches = 0;
+        for (DBuf* b : {&ws, &lws, &lquad}) b->release();
+        for (Team& t : team) t.quad.release();
+    }
+    // frees everything the plan holds, also when its creation stopped half way
+    ~fbc_plan_s() {
+        DevGuard dg_;
+        if (g.init) dg_.enter();
+        discard();
         for (DBuf* b : {&crp, &cadj, &cgid, &cbord, &segs, &units, &chunks, &bc, &bdist, &bsig, &ctr, &retry,
                         &bunits, &ws, &lquad, &lsegs, &lextra, &lunits, &lws})
             b->release();
@@ -968,6 +980,20 @@ int team_launch(const TeamCfg& c, const fbc::TeamParams& T) {
     return FBC_OK;
 }
 
+// The device memory of a team launch on the library's buffers that grows with the segments and units.
+int take_team(const Plan& P, const std::vector<Unit>& units) {
+    std::vector<char> seen(P.segs.size(), 0);
+    int64_t nq = 0;
+    for (const Unit& u : units)
+        if (!seen[u.seg]) {
+            seen[u.seg] = 1;
+            nq += P.segs[u.seg].n + P.seg_m[u.seg] / 3 + 1;
+        }
+    FBC_CK(g.tquad.ensure(sizeof(uint4) * (size_t)nq));
+    FBC_CK(g.tunits.ensure(sizeof(Unit) * units.size()));
+    return FBC_OK;
+}
+
 // A team launch on the library's buffers.
 template <class Prec>
 int launch_team(const Plan& P, std::vector<Unit>&& units, fbc_stats* st, int& launches) {
@@ -1002,9 +1028,12 @@ struct LogBuild {
     std::vector<fbc::LogQuads> list;
     std::vector<std::pair<uint4**, uint4*>> keep;  // a graph's, handed over once their build is launched
     int nmax = 0;
-    ~LogBuild() {
+    void drop() {
         for (auto& k : keep) cudaFree(k.second);
+        keep.clear();
+        list.clear();
     }
+    ~LogBuild() { drop(); }
 };
 int log_quads_prepare(Plan& P, const std::vector<char>& logs, DBuf& quads, LogBuild& b) {
     int64_t own = 0;
@@ -1063,6 +1092,7 @@ struct LogCfg {
     KernFn kern = nullptr;
     int threads = 0, teams = 0;
     int cluster = 1;          // blocks of a source (log_cluster_kernel)
+    int ws_n = 0;
     int64_t stride = 0, blocks = 0;
     std::vector<Unit> units;  // biggest segments first
 };
@@ -1145,22 +1175,28 @@ int log_config(const Plan& P, std::vector<Unit>&& units, int ws_n, int64_t budge
     int bps = 1;
     FBC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, c.kern, c.threads * c.teams, 0));
     const int64_t sb = fbc::lstate_bytes<Prec>(ws_n);
+    c.ws_n = ws_n;
     c.stride = (sb + 255) & ~int64_t(255);
     const int64_t want = std::min<int64_t>((int64_t)g.nsm * std::max(bps, 1), ((int64_t)c.units.size() + c.teams - 1) / c.teams);
     c.blocks = std::max<int64_t>(1, std::min<int64_t>(want, budget / (c.stride * c.teams)));
     return FBC_OK;
 }
 
-// A log-kernel launch on the library's workspace.
+// The device memory of a log launch on the library's workspace: the segments' quads and the slots.
 template <class Prec>
-int launch_log(const Plan& P, std::vector<Unit>&& units, fbc_stats* st, int& launches) {
-    if (units.empty()) return FBC_OK;
+int take_log(Plan& P, const std::vector<Unit>& units, const std::vector<char>& logs, LogBuild& b, LogCfg& c) {
     int ws_n = 0;
     for (const Unit& u : units) ws_n = std::max(ws_n, P.segs[u.seg].n);
-    LogCfg c;
-    Workspace& W = g.wsl;
-    FBC_TRY(log_config<Prec>(P, std::move(units), ws_n, ws_budget(&W), c));
-    FBC_CK(ws_take(W, c.blocks * c.teams * c.stride, false));
+    FBC_TRY(log_quads_prepare(P, logs, g.lquad, b));
+    FBC_TRY(log_config<Prec>(P, std::vector<Unit>(units), ws_n, ws_budget(&g.wsl), c));
+    FBC_CK(g.lunits.ensure(sizeof(Unit) * units.size()));
+    FBC_CK(ws_take(g.wsl, c.blocks * c.teams * c.stride, false));
+    return FBC_OK;
+}
+
+// A log-kernel launch on the library's workspace (take_log).
+int launch_log(const Plan& P, const LogCfg& c, fbc_stats* st, int& launches) {
+    if (c.units.empty()) return FBC_OK;
     FBC_CK(g.lunits.ensure(sizeof(Unit) * c.units.size()));
     FBC_CK(cudaMemcpyAsync(g.lunits.p, c.units.data(), sizeof(Unit) * c.units.size(), cudaMemcpyHostToDevice, g.st));
     if (st) st->h2d_bytes += (int64_t)(sizeof(Unit) * c.units.size());
@@ -1168,9 +1204,9 @@ int launch_log(const Plan& P, std::vector<Unit>&& units, fbc_stats* st, int& lau
     K.units = g.lunits.as<Unit>();
     K.nunits = (int64_t)c.units.size();
     K.next_unit = g.ctr.as<unsigned long long>() + 3;
-    K.ws = W.buf.as<char>();
+    K.ws = g.wsl.buf.as<char>();
     K.ws_stride = c.stride;
-    K.ws_n = ws_n;
+    K.ws_n = c.ws_n;
     // one segment with an output map: BC is summed in the segment's order and scattered once at the end
     const Seg& one = P.segs[c.units[0].seg];
     bool single = one.gid != nullptr;
@@ -1335,34 +1371,51 @@ int run_plan_t(Plan& P, fbc_stats* st) {
     }
     if (st)
         for (const Unit& u : P.units) st->retries += ties[u.seg];
-    int64_t nwarp = 0, nblock = 0;  // units of the two phases
-    double warp_bytes = 0, block_bytes = 0;
-    for (const Unit& u : P.units) {
-        if (logs[u.seg]) {
-            lg.push_back(u);
-            nblock += 1;
-            block_bytes += 40.0 * (double)P.seg_m[u.seg] + 52.0 * P.segs[u.seg].n;
-            continue;
+    for (const Unit& u : P.units)
+        (logs[u.seg] ? lg : !team[u.seg] ? rest : P.segs[u.seg].n <= g.opt.warp_max_n ? tw : tb).push_back(u);
+    // where device memory does not hold what the team and log kernels take, the older kernels, which need less
+    const auto instead = [&](std::vector<Unit>& v) {
+        (void)cudaGetLastError();
+        rest.insert(rest.end(), v.begin(), v.end());
+        v.clear();
+    };
+    LogBuild lb;
+    LogCfg lc;
+    if (!lg.empty()) {
+        const int rc = take_log<Prec>(P, lg, logs, lb, lc);
+        if (rc && rc != FBC_ERR_OOM) return rc;
+        if (rc) {
+            instead(lg);
+            lb.drop();
+            lc = LogCfg{};
+            g.lquad.release();
+            g.lunits.release();
         }
-        if (!team[u.seg]) {
-            rest.push_back(u);
-            continue;
-        }
-        const bool up_to = P.segs[u.seg].n <= g.opt.warp_max_n;
-        (up_to ? tw : tb).push_back(u);
-        (up_to ? nwarp : nblock) += 1;
-        (up_to ? warp_bytes : block_bytes) += 40.0 * (double)P.seg_m[u.seg] + 52.0 * P.segs[u.seg].n;
     }
-    for (std::vector<Unit>* v : {&tw, &tb})
+    for (std::vector<Unit>* v : {&tw, &tb}) {
         std::stable_sort(v->begin(), v->end(), [](const Unit& a, const Unit& b) { return a.seg < b.seg; });
+        const int rc = v->empty() ? FBC_OK : take_team(P, *v);
+        if (rc && rc != FBC_ERR_OOM) return rc;
+        if (!rc) continue;
+        instead(*v);
+        if (tw.empty()) {
+            g.tquad.release();
+            g.tunits.release();
+        }
+    }
     OldSplit sp;
     split_old(P, rest, sp);
-    nwarp += (int64_t)sp.uw.size();
-    nblock += (int64_t)sp.ub.size();
-    for (const Unit& u : sp.uw) warp_bytes += 40.0 * (double)P.seg_m[u.seg] + 52.0 * P.segs[u.seg].n;
-    for (const Unit& u : sp.ub) block_bytes += 40.0 * (double)P.seg_m[u.seg] + 52.0 * P.segs[u.seg].n;
-    LogBuild lb;
-    if (!lg.empty()) FBC_TRY(log_quads_prepare(P, logs, g.lquad, lb));
+    const int64_t nwarp = (int64_t)(tw.size() + sp.uw.size());  // units of the two phases
+    const int64_t nblock = (int64_t)(tb.size() + lg.size() + sp.ub.size());
+    double warp_bytes = 0, block_bytes = 0;
+    const auto bytes = [&](const std::vector<Unit>& v, double& b) {
+        for (const Unit& u : v) b += 40.0 * (double)P.seg_m[u.seg] + 52.0 * P.segs[u.seg].n;
+    };
+    bytes(tw, warp_bytes);
+    bytes(sp.uw, warp_bytes);
+    bytes(tb, block_bytes);
+    bytes(lg, block_bytes);
+    bytes(sp.ub, block_bytes);
     FBC_CK(g.segs.ensure(sizeof(Seg) * std::max<size_t>(P.segs.size(), 1)));
     FBC_CK(cudaMemcpyAsync(g.segs.p, P.segs.data(), sizeof(Seg) * P.segs.size(),
                            cudaMemcpyHostToDevice, g.st));
@@ -1378,7 +1431,7 @@ int run_plan_t(Plan& P, fbc_stats* st) {
         FBC_TRY(launch_team<Prec>(P, std::move(tb), st, launches));
     }
     FBC_TRY(log_quads_build(lb, g.segs.as<Seg>(), g.lsegs, g.lextra, launches));
-    FBC_TRY(launch_log<Prec>(P, std::move(lg), st, launches));
+    FBC_TRY(launch_log(P, lc, st, launches));
     FBC_TRY(launch_old_blocks<Prec>(P, sp, st, launches));
     for (auto& r : P.results) fbc_host::prefault(r.first, r.second);  // while the kernels run
     int err[2] = {0, 0};
@@ -3040,20 +3093,7 @@ int plan_widen(fbc_plan_s* p) {
             more = true;
         }
     if (!more) return FBC_OK;
-    for (int i = 0; i < 2; ++i) {
-        if (p->exec[i]) cudaGraphExecDestroy(p->exec[i]);
-        if (p->graph[i]) cudaGraphDestroy(p->graph[i]);
-        p->exec[i] = nullptr;
-        p->graph[i] = nullptr;
-    }
-    p->captured = false;
-    p->wbytes = p->bbytes = 0;
-    p->wunits = p->bunits_n = 0;
-    p->launches = 0;
-    // The new capture may lay the slots out differently (other communities, other free memory): the frontier
-    // kernel takes a slot whose header is not zero as one it has set up, so it starts from cleared ones again.
-    p->ws.release();
-    p->lws.release();
+    p->discard();
     struct Restore {
         Options now = g.opt;
         ~Restore() { g.opt = now; }
@@ -3102,8 +3142,17 @@ int fbc_cluster_plan_create(fbc_graph G, int32_t nclusters, const int64_t* coff,
     FBC_CK(cudaMallocHost(&p->h_bsig, e8));
     FBC_CK(cudaMallocHost(&p->h_ctl, 64));
     if (!P.units.empty()) {
-        if (precision == FBC_PREC_FP64) FBC_TRY(plan_capture<fbc::PrecF64>(p, P));
-        else FBC_TRY(plan_capture<fbc::PrecDF32>(p, P));
+        const auto capture = [&]() {
+            return precision == FBC_PREC_FP64 ? plan_capture<fbc::PrecF64>(p, P) : plan_capture<fbc::PrecDF32>(p, P);
+        };
+        int rc = capture();
+        if (rc == FBC_ERR_OOM && p->wide.empty()) {  // not enough device memory: the older kernels need less
+            (void)cudaGetLastError();
+            p->wide.assign((size_t)nclusters, 1);
+            p->discard();
+            rc = capture();
+        }
+        FBC_TRY(rc);
     }
     *out = guard.release();
     return FBC_OK;
