@@ -121,6 +121,14 @@ _COPIERS = min(16, os.cpu_count() or 1)
 _copy_pool: ThreadPoolExecutor | None = None
 
 
+def _forget_pool() -> None:
+    global _copy_pool
+    _copy_pool = None
+
+
+os.register_at_fork(after_in_child=_forget_pool)  # its threads are the parent's
+
+
 def _copy(a: np.ndarray) -> np.ndarray:
     """a.copy(), by several threads where it is large (the fresh pages' faults, not the bytes, take the
     time of one; NumPy copies without the interpreter lock)."""
@@ -129,10 +137,13 @@ def _copy(a: np.ndarray) -> np.ndarray:
     if a.nbytes < 8 << 20 or _COPIERS < 2:
         out[:] = a
         return out
-    if _copy_pool is None:
-        _copy_pool = ThreadPoolExecutor(_COPIERS)
     cut = np.linspace(0, a.size, _COPIERS + 1).astype(np.int64)
-    list(_copy_pool.map(lambda k: np.copyto(out[cut[k]:cut[k + 1]], a[cut[k]:cut[k + 1]]), range(_COPIERS)))
+    try:
+        if _copy_pool is None:
+            _copy_pool = ThreadPoolExecutor(_COPIERS)
+        list(_copy_pool.map(lambda k: np.copyto(out[cut[k]:cut[k + 1]], a[cut[k]:cut[k + 1]]), range(_COPIERS)))
+    except RuntimeError:  # no threads to be had, as when the interpreter is shutting down
+        out[:] = a
     return out
 
 
