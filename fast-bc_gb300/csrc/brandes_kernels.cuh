@@ -120,7 +120,7 @@ __device__ __forceinline__ void request_retry(const KParams& P, const Unit& u, i
 
 // More rounds than four times the root of n, when a source of the team and log kernels is looked at for narrow ones
 // (a road-like source has run two to three times the root by its end).
-__device__ __forceinline__ bool many_rounds(int n, int nr) { return (float)nr * (float)nr > 16.0f * (float)n; }
+__device__ __forceinline__ bool many_rounds(int n, int nr) { return nr > 46340 || nr * nr > 16 * n; }
 
 // Units of a segment of which more than a third came back (or were too narrow) are handed back unstarted: a unit given back
 // has cost its distances and counts, about 0.6 of its time here, and is done again by a kernel that takes

@@ -138,7 +138,7 @@ struct Ctx {
     Options opt;
     DBuf retry, segs, units_b, units_w, chunks, crp, cadj, cgid, cbord, bc, bdist, bsig, ctr, dbg, bcseg;
     // team kernel: segment list, quads, continuation counts, units and work items of its launches
-    DBuf tsegs, tquad, textra, tunits, tchunks;
+    DBuf tsegs, tquad, tunits, tchunks;
     // log kernel: quads of communities, the lists of a quad build, units
     DBuf lquad, lsegs, lextra, lunits;
     DBuf gave;  // per segment: units ended, units given back
@@ -210,7 +210,7 @@ struct fbc_plan_s {
     DBuf crp, cadj, cgid, cbord, segs, units, chunks, bc, bdist, bsig, ctr, retry, bunits, ws;
     DBuf lquad, lsegs, lextra, lunits, lws;  // log launch
     struct Team {  // one team launch: communities up to warp_max_n, and above it
-        DBuf segs, quad, extra, units, chunks;
+        DBuf segs, quad, units, chunks;
     } team[2];
     double* h_bc = nullptr;
     double* h_bdist = nullptr;
@@ -253,7 +253,7 @@ struct fbc_plan_s {
                         &bunits, &ws, &lquad, &lsegs, &lextra, &lunits, &lws})
             b->release();
         for (Team& t : team)
-            for (DBuf* b : {&t.segs, &t.quad, &t.extra, &t.units, &t.chunks}) b->release();
+            for (DBuf* b : {&t.segs, &t.quad, &t.units, &t.chunks}) b->release();
         if (h_bc) cudaFreeHost(h_bc);
         if (h_bdist) cudaFreeHost(h_bdist);
         if (h_bsig) cudaFreeHost(h_bsig);
@@ -935,20 +935,18 @@ void team_config(const Plan& P, std::vector<Unit>&& units, TeamCfg& c) {
 
 // Upload a team launch's lists into the given buffers and build its quads from the segments'
 // CSRs (dsegs: the uploaded segment list).
-int team_upload(TeamCfg& c, const Seg* dsegs, DBuf& tsegs, DBuf& tquad, DBuf& textra, DBuf& tunits, DBuf& tchunks,
+int team_upload(TeamCfg& c, const Seg* dsegs, DBuf& tsegs, DBuf& tquad, DBuf& tunits, DBuf& tchunks,
                 fbc_stats* st) {
     FBC_CK(tsegs.ensure(sizeof(fbc::TeamSeg) * c.segs.size()));
     FBC_CK(tquad.ensure(sizeof(uint4) * (size_t)c.nquads));
-    FBC_CK(textra.ensure(sizeof(int32_t) * c.segs.size()));
     FBC_CK(tunits.ensure(sizeof(Unit) * c.units.size()));
     FBC_CK(tchunks.ensure(sizeof(fbc::Chunk) * c.chunks.size()));
     for (size_t i = 0; i < c.segs.size(); ++i) c.segs[i].quad = tquad.as<uint4>() + c.quad_off[i];
     FBC_CK(cudaMemcpyAsync(tsegs.p, c.segs.data(), sizeof(fbc::TeamSeg) * c.segs.size(), cudaMemcpyHostToDevice, g.st));
     FBC_CK(cudaMemcpyAsync(tunits.p, c.units.data(), sizeof(Unit) * c.units.size(), cudaMemcpyHostToDevice, g.st));
     FBC_CK(cudaMemcpyAsync(tchunks.p, c.chunks.data(), sizeof(fbc::Chunk) * c.chunks.size(), cudaMemcpyHostToDevice, g.st));
-    FBC_CK(cudaMemsetAsync(textra.p, 0, sizeof(int32_t) * c.segs.size(), g.st));
     const dim3 grid((unsigned)c.segs.size(), (unsigned)std::max(1, std::min(64, (c.nmax + 255) / 256)));
-    fbc::team_quads_kernel<<<grid, 256, 0, g.st>>>(dsegs, tsegs.as<fbc::TeamSeg>(), textra.as<int32_t>());
+    fbc::team_quads_kernel<<<grid, 256, 0, g.st>>>(dsegs, tsegs.as<fbc::TeamSeg>());
     FBC_CK(cudaGetLastError());
     if (st)
         st->h2d_bytes += (int64_t)(sizeof(fbc::TeamSeg) * c.segs.size() + sizeof(Unit) * c.units.size() +
@@ -956,14 +954,13 @@ int team_upload(TeamCfg& c, const Seg* dsegs, DBuf& tsegs, DBuf& tquad, DBuf& te
     return FBC_OK;
 }
 
-fbc::TeamParams team_params(const TeamCfg& c, const KParams& base, DBuf& tsegs, DBuf& textra, DBuf& tunits,
+fbc::TeamParams team_params(const TeamCfg& c, const KParams& base, DBuf& tsegs, DBuf& tunits,
                             DBuf& tchunks, unsigned long long* next_chunk) {
     fbc::TeamParams T{};
     T.k = base;
     T.k.units = tunits.as<Unit>();
     T.k.nunits = (int64_t)c.units.size();
     T.tsegs = tsegs.as<fbc::TeamSeg>();
-    T.extra = textra.as<int32_t>();
     T.chunks = tchunks.as<fbc::Chunk>();
     T.nchunks = (int32_t)c.chunks.size();
     T.smem = (int32_t)team_dyn_smem();
@@ -1000,8 +997,8 @@ int launch_team(const Plan& P, std::vector<Unit>&& units, fbc_stats* st, int& la
     if (units.empty()) return FBC_OK;
     TeamCfg c;
     team_config(P, std::move(units), c);
-    FBC_TRY(team_upload(c, g.segs.as<Seg>(), g.tsegs, g.tquad, g.textra, g.tunits, g.tchunks, st));
-    FBC_TRY(team_launch<Prec>(c, team_params(c, base_params(P), g.tsegs, g.textra, g.tunits, g.tchunks,
+    FBC_TRY(team_upload(c, g.segs.as<Seg>(), g.tsegs, g.tquad, g.tunits, g.tchunks, st));
+    FBC_TRY(team_launch<Prec>(c, team_params(c, base_params(P), g.tsegs, g.tunits, g.tchunks,
                                              g.ctr.as<unsigned long long>() + 1)));
     launches += 2;
     return FBC_OK;
@@ -2164,7 +2161,7 @@ int fbc_gpu_shutdown(void) {
     cudaStreamSynchronize(g.st);
     for (DBuf* b : {&g.c_off, &g.c_id, &g.c_lid, &g.c_isb, &g.c_flag, &g.c_scan, &g.c_sums, &g.c_boff,
                     &g.c_bsrc, &g.c_m, &g.c_err, &g.retry, &g.segs, &g.units_b, &g.units_w, &g.chunks, &g.crp, &g.cadj, &g.cgid, &g.cbord, &g.bc,
-                    &g.bdist, &g.bsig, &g.ctr, &g.dbg, &g.bcseg, &g.tsegs, &g.tquad, &g.textra, &g.tunits, &g.tchunks, &g.lquad, &g.lsegs, &g.lextra, &g.lunits, &g.gave})
+                    &g.bdist, &g.bsig, &g.ctr, &g.dbg, &g.bcseg, &g.tsegs, &g.tquad, &g.tunits, &g.tchunks, &g.lquad, &g.lsegs, &g.lextra, &g.lunits, &g.gave})
         b->release();
     g.wsb.buf.release();
     g.wsw.buf.release();
@@ -3029,8 +3026,8 @@ int plan_capture(fbc_plan_s* p, Plan& P) {
         ++nteam;
         fbc_plan_s::Team& t = p->team[i];
         team_config(P, std::move(ut[i]), tc[i]);
-        FBC_TRY(team_upload(tc[i], p->segs.as<Seg>(), t.segs, t.quad, t.extra, t.units, t.chunks, nullptr));
-        T[i] = team_params(tc[i], base, t.segs, t.extra, t.units, t.chunks, p->ctr.as<unsigned long long>() + 4 + i);
+        FBC_TRY(team_upload(tc[i], p->segs.as<Seg>(), t.segs, t.quad, t.units, t.chunks, nullptr));
+        T[i] = team_params(tc[i], base, t.segs, t.units, t.chunks, p->ctr.as<unsigned long long>() + 4 + i);
         FBC_CK(cudaFuncSetAttribute(fbc::team_kernel<Prec>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T[i].smem));
     }
     LogCfg lc;

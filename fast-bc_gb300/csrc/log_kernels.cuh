@@ -19,8 +19,8 @@
 // counter, counts and pushes per Kahn level, device time, FP32C, one GB300: 280 pivots of the 2048x2048
 // grid 235.7 -> 180 ms; 1,309 pivots of the 256x256 grid 18.9 -> 14.0; the 16,384 sources of the 128x128
 // grid 47.3 -> 34.0; communities of 4.5K to 20K vertices (50K sources, FP64) 107 -> 82.
-// A source whose counts reach 2^24, whose distances outgrow a word, or with more rounds than are
-// kept stops before its dependencies and is done by the kernels with wider fields.
+// A source whose counts reach 2^24, whose distances outgrow a word, or of too many narrow rounds stops before its
+// dependencies and is done by the kernels with wider fields.
 #pragma once
 #include <cooperative_groups.h>
 #include "frontier_kernels.cuh"

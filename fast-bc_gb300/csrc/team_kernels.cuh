@@ -1,5 +1,5 @@
 // Batched schedule, segments of which shared memory holds two or more sources' state (up to some 8,400
-// vertices): a persistent kernel whose blocks pull (segment, chunk of sources) work items; the
+// vertices; one, up to 16,384, where there are at most four units an SM): a persistent kernel whose blocks pull (segment, chunk of sources) work items; the
 // block's warps form teams, one source per team, every word of a source's state in shared memory.
 //
 // What bounds it is the chain of dependent accesses of each round (a few hundred rounds per source)
@@ -12,12 +12,12 @@
 //     (1% more pops on road grids; the log's rounds outnumber the DAG's levels by a fifth);
 //   * 13.5 bytes of state per vertex, planes reused pass after pass:
 //       plane 0   (dist | stamp) word                    -> low word of the coefficient
-//       plane 1   log of the pops (16 bits, two per vertex; a pop that a later one replaces is cleared), and from
-//                 its far end the rounds' first log places
+//       plane 1   log of the pops (16 bits, two per vertex; a pop that a later one replaces is cleared), with the
+//                 rounds' first log places from its far end
 //       plane 2   log place of the last pop              -> path count (32 bits) -> high word
-//     an 8-bit tight-edge mask (16 bits for rows of 9 to 16 edges).
-//     Path counts stay below 2^24 here; a source that needs more, or more rounds than are kept, stops
-//     before its dependencies and is done by the kernels with wider counts;
+//     and an 8-bit tight-edge mask (16 bits for rows of 9 to 16 edges).
+//     Path counts stay below 2^24 here; a source that needs more, or has too many narrow rounds, stops
+//     before its dependencies and is done by another kernel;
 //   * no far pile: when a bucket is empty, the next bucket's vertices are found by a sweep over the words
 //     (four a lane), which costs less than keeping a second queue up to date;
 //   * the dependency pass keeps the coefficient c_w = (1 + delta_w) / sigma_w in the place of dist and
@@ -38,36 +38,36 @@
 // Measured against the one-warp kernel at 24 bytes per vertex (batched_kernels.cuh) and the frontier
 // kernel, device time of exact or community runs, FP32C, one GB300: 65,536 sources over 76 communities
 // of 68 to 2,448 vertices 19.9 -> 5.8 ms; 4,096 vertices 1.8 ms; 8,372 vertices 11.6 -> 8.4 ms;
-// 16,384 vertices (one source per SM would fit) 54.7 against 47.3 ms of the frontier kernel, hence
-// the limit at two sources.
+// all 16,384 sources of that many vertices (one source per SM) 54.7 against 47.3 ms of the frontier kernel and
+// 34 of the log kernel, hence the limit at two sources where there are many.
 #pragma once
 #include "batched_kernels.cuh"
 
 namespace fbc {
 
-constexpr int kTeamThreads = 640;  // 20 warps of up to 102 registers (1,024 threads spill or are no faster)
+constexpr int kTeamThreads = 640;  // 20 warps of up to 96 registers (1,024 threads spill or are no faster)
 constexpr int kTeamMax = 15;          // teams of several warps in a block (named barriers 1..15)
 constexpr int kTeamRow = 16;          // longest row (mask bits)
-constexpr int kTeamIndeg = 255;       // most in-edges of a vertex (8-bit tight in-edge counts)
+constexpr int kTeamIndeg = 255;       // most in-edges of a vertex (sums of that many counts below 2^24 fit 32 bits)
 constexpr int kTeamDistBits = 24;     // most distance bits of a word (eight or more stamp bits)
 constexpr uint32_t kNoEdge = 0xffffffffu;    // an empty place of a quad (negative, as a link is)
 constexpr uint32_t kLink = 0x80010000u;      // | index of the row's next quad
 constexpr uint32_t kNoVertex = 0xffffu;
 constexpr int kTeamMaxN = 16384;      // 4 * vertex in 16 bits
 
-// Rows of a segment as quads: n first quads, then the continuations (`extra` of them).
+// Rows of a segment as quads: n first quads, then the continuations (`extra` of them, counted as they are built;
+// 0 before).
 struct TeamSeg {
     uint4* quad;
     int32_t seg;        // index into KParams::segs
     int32_t stamp_bits; // low bits of a word
     int32_t wide_mask;  // 16-bit masks (rows of more than 8 edges)
-    int32_t pad;
+    int32_t extra;
 };
 
 struct TeamParams {
     KParams k;
     const TeamSeg* tsegs;
-    const int32_t* extra;     // continuation quads of each team segment
     const Chunk* chunks;      // Chunk::seg indexes tsegs
     int32_t nchunks;
     int32_t smem;             // dynamic shared memory of a block (bytes)
@@ -75,16 +75,16 @@ struct TeamParams {
 };
 
 __host__ __device__ inline int64_t team_n16(int64_t n) { return (n + 15) & ~int64_t(15); }
-// shared-memory state of one source: beside the log room for n / 4 rounds; more (narrow sources) lie in its end
-__host__ __device__ inline int team_round_bytes(int64_t n16) { return (int)al16(n16 / 2 + 130); }
-__host__ __device__ inline int64_t team_rounds(int64_t n16) { return n16 / 2 + 256; }  // kept rounds
+// shared-memory state of one source: the log has room for two pops a vertex and n / 4 rounds' starts, which lie in
+// what the pops leave of it, so that narrow sources of more rounds fit (4 x 500 vertices, all sources, 5.8 -> 2.4 ms)
+__host__ __device__ inline int64_t team_log_bytes(int64_t n16) { return 4 * n16 + al16(n16 / 2 + 130); }
 __host__ __device__ inline int64_t team_bytes(int64_t n, bool wide_mask) {
-    return (wide_mask ? 14 : 13) * team_n16(n) + team_round_bytes(team_n16(n));
+    return (wide_mask ? 10 : 9) * team_n16(n) + team_log_bytes(team_n16(n));
 }
 
 // Quads of the team segments, one grid row of blocks per segment: the rows in their order, a row
 // of more than four edges continued in quads taken from the segment's counter.
-__global__ void team_quads_kernel(const Seg* __restrict__ segs, const TeamSeg* __restrict__ ts, int32_t* extra) {
+__global__ void team_quads_kernel(const Seg* __restrict__ segs, TeamSeg* ts) {
     const TeamSeg t = ts[blockIdx.x];
     const Seg sg = segs[t.seg];
     uint32_t* const q32 = reinterpret_cast<uint32_t*>(t.quad);
@@ -105,7 +105,7 @@ __global__ void team_quads_kernel(const Seg* __restrict__ segs, const TeamSeg* _
             e += k;
             int next = -1;
             if (left > 4) {
-                next = sg.n + atomicAdd(extra + blockIdx.x, 1);
+                next = sg.n + atomicAdd(&ts[blockIdx.x].extra, 1);
                 r[3] = kLink | (uint32_t)next;
             }
             reinterpret_cast<uint4*>(q32)[at] = make_uint4(r[0], r[1], r[2], r[3]);
@@ -256,16 +256,16 @@ struct CoefBits<float2> {
     }
 };
 
-// Whether a source is too narrow for the kernel after nr rounds of e pops together: more rounds to come than are
-// kept; and, where there are several waves of units (so that most of the segment's are then not begun), rounds that
-// the block's few sources cannot fill.  All sources, this kernel against those of the frontier kernel, ms: 10 x 700
+// Whether a source is too narrow for the kernel after nr rounds of e pops together: one or two vertices a round, as on
+// a path (all sources of one of 1,500 vertices: 6.8 ms, 9.9 with a bound on the rounds instead, which only the outer
+// sources meet, and late); and, where there are several waves of units (so that most of the segment's are then not
+// begun), rounds that the block's few sources cannot fill.  All sources, this kernel / the frontier kernel, ms: 10 x 700
 // vertices (two at once on an SM, 12 to 22 pops a round) 36.2 / 26.9, 5 x 1,000 (three; 6 to 11) 33.7 / 21.6; but
 // 16 x 350 (16 to 28) 11.2 / 12.8, 12 x 340 6.5 / 9.4, 8 x 500 (four; 9 to 15) 9.0 / 11.3.
 constexpr int kTeamMany = 16;  // units a block
 __device__ __forceinline__ bool team_narrow(const KParams& K, int n, int nr, int e) {
-    const float left = (float)n * (float)nr / (float)e;  // rounds that n pops take at this pace
-    return left > 0.9f * (float)team_rounds(team_n16(n)) ||
-           (K.gave && K.nunits > kTeamMany * (int64_t)gridDim.x && (float)n * left > 2e6f);
+    return (n > 512 && 20 * e < 41 * nr) || (K.gave && K.nunits > kTeamMany * (int64_t)gridDim.x &&
+                                             (float)n * (float)n * (float)nr > 2e6f * (float)e);
 }
 
 template <class Prec, bool kWarp, bool kRows>
@@ -275,16 +275,13 @@ __device__ __forceinline__ void TeamUnit<Prec, kWarp, kRows>::run(const KParams&
     const int n16 = (int)team_n16(n);
     char* const base = team_smem + off;
     uint32_t* const word = (uint32_t*)base;                // plane 0
-    const int rb = team_round_bytes(n16);
-    uint32_t* const sig = (uint32_t*)(base + 8 * n16 + rb);  // plane 2
+    uint32_t* const sig = (uint32_t*)(base + 4 * n16);     // plane 2
     const bool wide = ts.wide_mask != 0;
-    // addresses: planes 0 and 2, the log (plane 1, 2 * n16 pops and what the rounds leave of theirs), the first
-    // round's start (the next ones' below it), where a vertex was popped last (plane 2 in the distance pass),
-    // tight-edge masks
-    const uint32_t aword = smem_addr(base), alog = aword + 4u * (uint32_t)n16,
-                   arnd = alog + 4u * (uint32_t)n16 + (uint32_t)rb - 2u, asig = arnd + 2u, alast = asig,
-                   amask = asig + 4u * (uint32_t)n16, amask2 = amask + (uint32_t)n16;
-    const int rndcap = (int)team_rounds(n16);
+    // addresses: planes 0 and 2, where a vertex was popped last (plane 2 in the distance pass), tight-edge masks,
+    // the log (plane 1), the first round's start at its end (the next ones' below it)
+    const uint32_t aword = smem_addr(base), asig = aword + 4u * (uint32_t)n16, alast = asig,
+                   amask = aword + 8u * (uint32_t)n16, amask2 = amask + (uint32_t)n16,
+                   alog = amask + (wide ? 2u : 1u) * (uint32_t)n16, arnd = alog + (uint32_t)team_log_bytes(n16) - 2u;
     const int sb = ts.stamp_bits;
     const uint32_t smask = (1u << sb) - 1u, one = 1u << sb;
     const int dinf = (int)(kNoEdge >> sb);                 // unreached: all distance bits set
@@ -313,6 +310,7 @@ __device__ __forceinline__ void TeamUnit<Prec, kWarp, kRows>::run(const KParams&
         uint32_t stamp = smask;
         int left = (int)min((int64_t)K.iter_mult * ((int64_t)n + 2), (int64_t)kInf);  // steps left
         nr = 0;
+        uint32_t logend = arnd;  // the next round's start, and the end of the log's free places
         bool full = false;
         for (;;) {
             const int cs = c3;
@@ -333,9 +331,9 @@ __device__ __forceinline__ void TeamUnit<Prec, kWarp, kRows>::run(const KParams&
                     stamp = smask;
                     sync();
                 }
-                if (nr == rndcap) { bad = kErrNarrow; break; }
                 const uint32_t st = --stamp;
-                if (tid == 0) sts16(arnd - 2u * (uint32_t)nr, (uint32_t)s);
+                if (tid == 0) sts16(logend, (uint32_t)s);
+                logend -= 2u;
                 ++nr;
                 for (int b = s + (tid & ~31); b < e; b += nth) {
                     const int i = b + lane;
@@ -363,7 +361,7 @@ __device__ __forceinline__ void TeamUnit<Prec, kWarp, kRows>::run(const KParams&
                             const uint32_t old = atom_min_ge0(a, aword + x4[t], key);
                             want[t] = near && key < old && (old & smask) != st;
                         }
-                        push(want, x4, alog + 2u * (uint32_t)e, arnd - 2u * (uint32_t)nr, nn, cnt);
+                        push(want, x4, alog + 2u * (uint32_t)e, logend, nn, cnt);
                         const bool link = quad_linked(q);
                         if (!__any_sync(kFull, link)) break;
                         const uint32_t next = link ? 4u * (q.w & 0xffffu) : v4;
@@ -388,7 +386,7 @@ __device__ __forceinline__ void TeamUnit<Prec, kWarp, kRows>::run(const KParams&
                         want[t] = d >= T0 && d < T;
                         if (d >= T) dmin = min(dmin, d);
                     }
-                    push(want, x4, alog + 2u * (uint32_t)e, arnd - 2u * (uint32_t)nr, nn, cnt);
+                    push(want, x4, alog + 2u * (uint32_t)e, logend, nn, cnt);
                 }
                 dmin = __reduce_min_sync(kFull, dmin);
                 if constexpr (!kWarp) {
@@ -404,16 +402,17 @@ __device__ __forceinline__ void TeamUnit<Prec, kWarp, kRows>::run(const KParams&
             }
             s = e;
             e += nn;
-            if (alog + 2u * (uint32_t)e > arnd - 2u * (uint32_t)nr) { full = true; break; }
+            if (alog + 2u * (uint32_t)e > logend) { full = true; break; }
         }
         sync();
         total = e;
         if (!full) break;
-        // more than two pops a vertex: again with narrower buckets (width 1 pops every vertex once)
+        // the log is full: again with narrower buckets (width 1 pops every vertex once, and there is room for
+        // that and as many rounds)
         delta = max(1, delta >> 2);
     }
-    if (tid == 0 && !bad && many_rounds(n, nr) && team_narrow(K, n, nr, total)) count_narrow(K, u.seg);
 
+    if (tid == 0 && !bad && many_rounds(n, nr) && team_narrow(K, n, nr, total)) count_narrow(K, u.seg);
     if (!bad) {
         // --------------------------------------------------------------- path counts
         // round by round over the last pops (every tight predecessor's is in an earlier round):
@@ -599,7 +598,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) team_kernel(TeamParams TP) {
         const Chunk ch = TP.chunks[ci];
         const TeamSeg ts = TP.tsegs[ch.seg];
         const Seg sg = TP.k.segs[ts.seg];
-        const int nq = sg.n + TP.extra[ch.seg];
+        const int nq = sg.n + ts.extra;
         const TeamSplit sp = team_split(sg.n, nq, ts.wide_mask != 0, TP.smem, ch.count, nw);
         if (sp.rows)
             for (int i = threadIdx.x; i < nq; i += blockDim.x)
