@@ -30,8 +30,8 @@
 //     computed in its arithmetic -- none where there is one such member.
 // A cluster of up to eight blocks shares a set's points, because the sets are few and of very
 // different sizes; distances are summed in 32 bits where the set's range allows it.  20 communities of
-// a 108x108 grid (143 to 1,557 points, 45 to 124 borders): a call of 631 ms
-// with one block per set and none of this takes 5.7 (4.4 on the device, 723 before; 2.9 of 9.2 million cycles of
+// a 108x108 grid (143 to 1,557 points, 45 to 124 borders): a call of 739 ms
+// with one block per set and none of this takes 5.0 (on the device 735 and 4.1; 2.9 of 9.2 million cycles of
 // the largest set are its 777 initialisation steps, each a choice among all its blocks).
 #pragma once
 #include <cooperative_groups.h>

@@ -89,7 +89,7 @@ const char* fbc_last_error_string(void);
  *   "frontier_threads" block size of the frontier kernel (32..128; above 128 the wide form)
  *                      (the frontier kernel runs what the team and log kernels do not take: rows of more
  *                      than 16 edges, in-degrees above 255, weights outside 8..255 where the state is not
- *                      in shared memory -- and everything above warp_max_n where "group" forces it)
+ *                      in shared memory, graphs rich in equally long ways -- and everything above warp_max_n where "group" forces it)
  *   "group"            0 = automatic; 1, 2, 4: segments above warp_max_n run on the frontier kernel with
  *                      that many sources per block (others refused)
  *   "chunk_max"        sources per work item of the shared-memory kernels
