@@ -270,7 +270,32 @@ int check_init(DevGuard& dg) {
     return FBC_OK;
 }
 
-// The graph's ties, from a sample of its uploaded rows (waits for the stream).
+// What a sample of the uploaded rows says of a graph's ties (gb_ties_kernel).  Where path counts could grow with them
+// (tie_rich), a few searches tell whether the graph is as deep as one in a plane; if not, its paths are too short for
+// that (a ring of 4,000 vertices with 10% shortcuts and one weight: all sources 1.5 ms in the team kernel, 4.8
+// in the older ones).
+constexpr double kTieShare = 0.02, kTieMost = 8.0, kTieMostOne = 64.0;
+constexpr double kPlaneHops = 1.6;  // times the hops for four times the vertices (planes 1.8 and more, that ring 1.3)
+cudaError_t set_ties(fbc_graph_s* G, int tied, int seen) {
+    G->ties = seen > 0 ? (double)tied / (double)seen : 0.0;
+    if (G->ties < kTieShare || G->ties * G->ties * (double)G->n * (double)G->n < kTieMost * (double)G->m) return cudaSuccess;
+    cudaError_t e = g.ctr.ensure(64);
+    if (e != cudaSuccess) return e;
+    static_assert(2 * fbc::kBallStarts * sizeof(int) <= 64, "");
+    const int many = std::max(2, std::min(fbc::kBallMost, G->n / 2));
+    int h[2 * fbc::kBallStarts] = {};
+    fbc::gb_ball_kernel<<<fbc::kBallStarts, 256, 0, g.st>>>(G->n, G->d_rp, G->d_adj, std::max(1, many / 4), many, g.ctr.as<int>());
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, g.ctr.p, sizeof(h), cudaMemcpyDeviceToHost, g.st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(g.st);
+    int h1 = 0, h2 = 0;
+    for (int i = 0; i < fbc::kBallStarts; ++i) {
+        h1 += h[2 * i];
+        h2 += h[2 * i + 1];
+    }
+    if (h2 > 0 && (double)h2 < kPlaneHops * (double)h1) G->ties = 0.0;
+    return e;
+}
 cudaError_t graph_ties(fbc_graph_s* G) {
     cudaError_t e = g.ctr.ensure(64);
     if (e == cudaSuccess) e = cudaMemsetAsync(g.ctr.p, 0, 64, g.st);
@@ -281,8 +306,7 @@ cudaError_t graph_ties(fbc_graph_s* G) {
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(t, d, sizeof(t), cudaMemcpyDeviceToHost, g.st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(g.st);
-    G->ties = t[0] > 0 ? (double)t[1] / (double)t[0] : 0.0;
-    return e;
+    return e == cudaSuccess ? set_ties(G, t[1], t[0]) : e;
 }
 
 // Validate a host CSR with double weights and build the device graph.
@@ -866,16 +890,18 @@ bool team_fits(const Plan& P, size_t s, int64_t units) {
 // the hops across the segment, about the root of its vertices over their edges: counts grow with the ties on the
 // way.  Such units would be run, given back and done again, so they start with the kernels of wider counts.  Share
 // squared x vertices / edges a vertex, and what came back (all sources, 2,432 of geometric graphs above 10,000
-// vertices): geometric graphs (3-NN) of 8,192 vertices 3.0: none, 16,000 7.7: half; 6-NN of 8,000 5.9: 11%; grids
-// of one weight 14 x 14 5.6: none, 16 x 16 7.3: 16%, 18 x 18 9.2: 40%, 30 x 30 25: all; of two weights 30 x 30
-// 3.5: none, 90 x 71 23: all; of weights to 8 90 x 71 1.4: none.  Device time with the units begun here and in the
-// older kernels at once: 6-NN 25.1 against 49.6 ms; geometric 16,000 16.6 / 15.7; 18 x 18 0.82 / 0.74; 30 x 30
-// 1.03 / 0.91; 8 x 500 10.1 / 9.2; 4 x 500 8.2 / 6.4.  Below the least share, ties are too few to multiply (road
-// weights of 1 to 100 on four million vertices: 0.0025, 6.6, none).
-constexpr double kTieShare = 0.02, kTieMost = 7.0;
-bool tie_rich(const Plan& P, size_t s) {
-    const double t = P.seg_ties[s], n = P.segs[s].n;
-    return t >= kTieShare && t * t * n * n >= kTieMost * (double)P.seg_m[s];
+// vertices): geometric graphs (3-NN) of 8,192 vertices 3.4: none, 12,000 5.5: 1%, 15,000 7.4: 3 to 11%, 16,000 8.6:
+// half; 6-NN of 8,000 5.9: 11%; of one weight, 3-NN of 2,000 vertices 8.2: 1 to 6%, grids of 14 x 14 5.6: none, 16 x 16
+// 7.3: 16%, 18 x 18 9.2: 40%, 30 x 30 25: all; grids of two weights 30 x 30 3.5: none, 90 x 71 23: all; of weights to 8
+// 90 x 71 1.4: none.  Device time with the units begun here / in the older kernels at once, ms: 6-NN 25.1 / 49.6;
+// geometric 15,000 12.7 / 14.1, 16,000 16.6 / 15.7; 16 x 16 0.53 / 0.62, 18 x 18 0.82 / 0.74, 30 x 30 1.03 / 0.91; 2,000 of
+// one weight 2.40 / 1.84; 8 x 500 10.1 / 9.2.  Below the least share, ties are too few to multiply (road weights of 1 to
+// 100 on four million vertices: 0.0025, 6.6, none).  Few sources (up to one an SM) cost little
+// where they come back (30 x 30 0.26 / 0.31 ms) and much where they would not have (geometric 16,000 0.97 / 2.58), so only
+// well above the line they start elsewhere (4 x 500, 57: 0.61 / 2.0; 8 x 500, 113: 3.4 / 2.1; 100 x 100, 279: 3.4 / 2.1).
+bool tie_rich(const Plan& P, size_t s, int64_t units) {
+    const double t = P.seg_ties[s], n = P.segs[s].n, most = units <= g.nsm ? kTieMostOne : kTieMost;
+    return t >= kTieShare && t * t * n * n >= most * (double)P.seg_m[s];
 }
 
 // Segments above warp_max_n go to the team kernel too, unless an option asks for the frontier
@@ -1362,7 +1388,7 @@ int run_plan_t(Plan& P, fbc_stats* st) {
             const bool up_to = P.segs[s].n <= std::min<int64_t>(g.opt.warp_max_n, 65535);
             team[s] = (up_to || blocks) && team_fits(P, s, (int64_t)P.units.size());
             logs[s] = !team[s] && !up_to && blocks && log_fits(P, s);
-            ties[s] = (team[s] || logs[s]) && tie_rich(P, s);
+            ties[s] = (team[s] || logs[s]) && tie_rich(P, s, (int64_t)P.units.size());
             if (ties[s]) team[s] = logs[s] = 0;
         }
     }
@@ -1897,12 +1923,13 @@ int device_csr_build(int64_t count, const int32_t* dsrc, const int32_t* ddst, co
     G->maxw = hi[2];
     G->maxindeg = hi[3];
     G->maxdeg = hi[6];
-    G->ties = hi[8] > 0 ? (double)hi[9] / (double)hi[8] : 0.0;
     G->meanw = medges ? (double)sumw / (double)medges : 1.0;
     if ((double)n * (double)G->maxw > 2147483646.0) {
         drop();
         return fail(FBC_ERR_RANGE, "n * max_weight exceeds the int32 distance range");
     }
+    e = set_ties(G, hi[9], hi[8]);
+    if (e != cudaSuccess) { drop(); return fail(FBC_ERR_CUDA, std::string("graph build: ") + cudaGetErrorString(e)); }
     G->host_ok = false;  // the host copy is fetched when something needs it
     *out = guard.release();
     return FBC_OK;
@@ -2563,7 +2590,7 @@ int fbc_single_source(fbc_graph G, int32_t source, int precision, double* out_de
     P.seg_ties.push_back(G->ties);
     P.units.push_back(Unit{0, source, 1.0, -1});
     P.bc_len = G->n;
-    P.sched = team_takes_blocks() && (team_fits(P, 0, 1) || log_fits(P, 0)) && !tie_rich(P, 0) ? FBC_SCHED_BATCHED : FBC_SCHED_PLAIN;
+    P.sched = team_takes_blocks() && (team_fits(P, 0, 1) || log_fits(P, 0)) && !tie_rich(P, 0, 1) ? FBC_SCHED_BATCHED : FBC_SCHED_PLAIN;
     P.results.emplace_back(out_dep, sizeof(double) * (size_t)G->n);
     int rc = run_plan(P, st);
     if (!rc) rc = download_bc(out_dep, G->n, false, st);

@@ -167,6 +167,58 @@ __global__ void __launch_bounds__(32 * kTieWarps) gb_ties_kernel(int32_t n, cons
     }
 }
 
+// Hops in which a search from a vertex (one a block) has met `few` and `many` vertices (0: never): in a plane four
+// times the vertices take about twice the hops, in a small world a few more.  Along the first kTieRow edges of a row.
+constexpr int kBallMost = 2048;   // `many` at most
+constexpr int kBallQueue = 3072;
+constexpr int kBallTable = 8192;  // vertices met, hashed
+constexpr int kBallHops = 256;
+constexpr int kBallStarts = 4;
+__global__ void __launch_bounds__(256) gb_ball_kernel(int32_t n, const int32_t* __restrict__ rp, const int2* __restrict__ adj,
+                                                      int few, int many, int* hops) {
+    __shared__ int table[kBallTable], queue[kBallQueue], cnt;
+    const int u = (int)((int64_t)(blockIdx.x + 1) * n / (kBallStarts + 1));
+    for (int i = threadIdx.x; i < kBallTable; i += blockDim.x) table[i] = -1;
+    __syncthreads();
+    const auto slot = [](int x) { return (int)(((unsigned)x * 2654435761u) >> 19); };  // (13 bits)
+    if (threadIdx.x == 0) {
+        table[slot(u)] = u;
+        queue[0] = u;
+        cnt = 1;
+    }
+    __syncthreads();
+    int lo = 0, hi = 1, h1 = 0, h2 = 0;
+    for (int hop = 1; hop <= kBallHops; ++hop) {
+        for (int i = lo + (int)threadIdx.x; i < hi; i += blockDim.x) {
+            const int v = queue[i], e0 = rp[v], e1 = min(rp[v + 1], e0 + kTieRow);
+            for (int e = e0; e < e1 && *(volatile int*)&cnt < kBallQueue; ++e) {
+                const int x = adj[e].x;
+                int s = slot(x);
+                for (int p = 0; p < 64; ++p, s = (s + 1) & (kBallTable - 1)) {
+                    const int old = atomicCAS(table + s, -1, x);
+                    if (old == -1) {
+                        const int at = atomicAdd(&cnt, 1);
+                        if (at < kBallQueue) queue[at] = x;
+                    }
+                    if (old == -1 || old == x) break;
+                }
+            }
+        }
+        __syncthreads();
+        const int met = min(cnt, kBallQueue);
+        __syncthreads();
+        if (!h1 && met >= few) h1 = hop;
+        if (met >= many) h2 = hop;
+        if (h2 || met == hi) break;
+        lo = hi;
+        hi = met;
+    }
+    if (threadIdx.x == 0) {
+        hops[2 * blockIdx.x] = h2 ? h1 : 0;
+        hops[2 * blockIdx.x + 1] = h2;
+    }
+}
+
 // The CSR in the caller's types: 64-bit offsets, destinations, weights as doubles (each null: not wanted).
 __global__ void gb_export_kernel(int32_t n, int64_t m, const int32_t* __restrict__ rp, const int2* __restrict__ adj,
                                  int64_t* __restrict__ rp64, int32_t* __restrict__ col, double* __restrict__ w) {
