@@ -179,7 +179,7 @@ struct fbc_graph_s {
     int32_t maxw = 0;
     int32_t maxindeg = 0;
     int32_t maxdeg = 0;  // longest row
-    double ties = 0.0;   // share of the vertices within two edges that have several shortest ways (gb_ties_kernel)
+    double ties = -1.0;  // share of the vertices within two edges that have several shortest ways (ties_of)
     double meanw = 1.0;
     int32_t* d_rp = nullptr;
     int2* d_adj = nullptr;
@@ -296,6 +296,7 @@ cudaError_t set_ties(fbc_graph_s* G, int tied, int seen) {
     if (h2 > 0 && (double)h2 < kPlaneHops * (double)h1) G->ties = 0.0;
     return e;
 }
+// The graph's ties, found out when a batched call first asks (some 20 us).
 cudaError_t graph_ties(fbc_graph_s* G) {
     cudaError_t e = g.ctr.ensure(64);
     if (e == cudaSuccess) e = cudaMemsetAsync(g.ctr.p, 0, 64, g.st);
@@ -307,6 +308,13 @@ cudaError_t graph_ties(fbc_graph_s* G) {
     if (e == cudaSuccess) e = cudaMemcpyAsync(t, d, sizeof(t), cudaMemcpyDeviceToHost, g.st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(g.st);
     return e == cudaSuccess ? set_ties(G, t[1], t[0]) : e;
+}
+int ties_of(const fbc_graph_s* G, int sched, double& t) {
+    t = 0.0;
+    if (sched != FBC_SCHED_BATCHED || G->m == 0) return FBC_OK;
+    if (G->ties < 0.0) FBC_CK(graph_ties(const_cast<fbc_graph_s*>(G)));
+    t = G->ties;
+    return FBC_OK;
 }
 
 // Validate a host CSR with double weights and build the device graph.
@@ -366,9 +374,8 @@ int make_graph(int32_t n, std::vector<int64_t>&& rp, std::vector<int32_t>&& col,
                                      cudaMemcpyHostToDevice, g.st);
     cudaError_t e4 = cudaMemcpyAsync(G->d_adj, adj.data(), sizeof(int2) * adj.size(),
                                      cudaMemcpyHostToDevice, g.st);
-    cudaError_t e5 = graph_ties(G);
+    cudaError_t e5 = cudaStreamSynchronize(g.st);
     if (e3 != cudaSuccess || e4 != cudaSuccess || e5 != cudaSuccess) {
-        cudaStreamSynchronize(g.st);
         cudaFree(G->d_rp);
         cudaFree(G->d_adj);
         delete G;
@@ -1794,7 +1801,8 @@ int prepare_clusters(const fbc_graph_s* G, int32_t nclusters, const int64_t* cof
         P.seg_maxw.push_back(G->maxw);
         P.seg_maxindeg.push_back(G->maxindeg);
         P.seg_maxdeg.push_back(G->maxdeg);
-        P.seg_ties.push_back(G->ties);
+        P.seg_ties.push_back(0.0);
+        FBC_TRY(ties_of(G, sched, P.seg_ties.back()));
         for (int32_t i = 0; i < s.n; ++i) P.units.push_back(Unit{c, i, 1.0, ent + (int64_t)i * s.nb});
         ent += (int64_t)s.n * s.nb;
     }
@@ -1846,8 +1854,8 @@ int device_csr_build(int64_t count, const int32_t* dsrc, const int32_t* ddst, co
     TmpBuf ints, deg, rs, cursor, keys, ndeg, indeg;
     FBC_CK(ints.ensure(64));
     // ints: [0] max source, [1] error bits, [2] max weight, [3] max in-degree, [4..5] weight sum,
-    // [6] longest row, [8] vertices within two edges of a sample, [9] tied ones
-    int hi[10] = {-1, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+    // [6] longest row
+    int hi[7] = {-1, 0, 0, 0, 0, 0, 0};
     FBC_CK(cudaMemcpyAsync(ints.p, hi, sizeof(hi), cudaMemcpyHostToDevice, g.st));
     int* di = ints.as<int>();
     fbc::gb_check_kernel<<<grid_for(count), 256, 0, g.st>>>(count, dsrc, ddst,
@@ -1911,7 +1919,6 @@ int device_csr_build(int64_t count, const int32_t* dsrc, const int32_t* ddst, co
                                                         dw, G->d_rp, G->d_adj, indeg.as<int32_t>(),
                                                         di + 2, (unsigned long long*)(di + 4), di + 6, di + 1);
     fbc::gb_max_kernel<<<grid_for(n), 256, 0, g.st>>>(n, indeg.as<int32_t>(), di + 3);
-    fbc::gb_ties_kernel<<<fbc::kTieSamples / fbc::kTieWarps, 32 * fbc::kTieWarps, 0, g.st>>>(n, G->d_rp, G->d_adj, di + 8, di + 9);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(hi, ints.p, sizeof(hi), cudaMemcpyDeviceToHost, g.st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(g.st);
@@ -1928,8 +1935,6 @@ int device_csr_build(int64_t count, const int32_t* dsrc, const int32_t* ddst, co
         drop();
         return fail(FBC_ERR_RANGE, "n * max_weight exceeds the int32 distance range");
     }
-    e = set_ties(G, hi[9], hi[8]);
-    if (e != cudaSuccess) { drop(); return fail(FBC_ERR_CUDA, std::string("graph build: ") + cudaGetErrorString(e)); }
     G->host_ok = false;  // the host copy is fetched when something needs it
     *out = guard.release();
     return FBC_OK;
@@ -2514,7 +2519,8 @@ int fbc_exact_bc(fbc_graph G, int precision, int sched, double* out_bc, fbc_stat
     P.seg_maxw.push_back(G->maxw);
     P.seg_maxindeg.push_back(G->maxindeg);
     P.seg_maxdeg.push_back(G->maxdeg);
-    P.seg_ties.push_back(G->ties);
+    P.seg_ties.push_back(0.0);
+    FBC_TRY(ties_of(G, sched, P.seg_ties.back()));
     for (int32_t s = 0; s < G->n; ++s) P.units.push_back(Unit{0, s, 1.0, -1});
     P.bc_len = G->n;
     P.results.emplace_back(out_bc, sizeof(double) * (size_t)G->n);
@@ -2549,7 +2555,8 @@ int fbc_sssp_dependency_batch(fbc_graph G, int64_t count, const int32_t* sources
     P.seg_maxw.push_back(G->maxw);
     P.seg_maxindeg.push_back(G->maxindeg);
     P.seg_maxdeg.push_back(G->maxdeg);
-    P.seg_ties.push_back(G->ties);
+    P.seg_ties.push_back(0.0);
+    FBC_TRY(ties_of(G, sched, P.seg_ties.back()));
     for (int64_t i = 0; i < count; ++i)
         P.units.push_back(Unit{0, map ? map[sources[i]] : sources[i], cards ? cards[i] : 1.0, -1});
     // on a relabelled graph, sources in the locality order: the sources running at once then
@@ -2587,7 +2594,8 @@ int fbc_single_source(fbc_graph G, int32_t source, int precision, double* out_de
     P.seg_maxw.push_back(G->maxw);
     P.seg_maxindeg.push_back(G->maxindeg);
     P.seg_maxdeg.push_back(G->maxdeg);
-    P.seg_ties.push_back(G->ties);
+    P.seg_ties.push_back(0.0);
+    FBC_TRY(ties_of(G, FBC_SCHED_BATCHED, P.seg_ties.back()));
     P.units.push_back(Unit{0, source, 1.0, -1});
     P.bc_len = G->n;
     P.sched = team_takes_blocks() && (team_fits(P, 0, 1) || log_fits(P, 0)) && !tie_rich(P, 0, 1) ? FBC_SCHED_BATCHED : FBC_SCHED_PLAIN;
@@ -3269,7 +3277,8 @@ int fbc_multi_exact_bc(int32_t ngraphs, const fbc_graph* graphs, int precision, 
         P.seg_maxw.push_back(graphs[i]->maxw);
         P.seg_maxindeg.push_back(graphs[i]->maxindeg);
         P.seg_maxdeg.push_back(graphs[i]->maxdeg);
-        P.seg_ties.push_back(graphs[i]->ties);
+        P.seg_ties.push_back(0.0);
+        FBC_TRY(ties_of(graphs[i], sched, P.seg_ties.back()));
         for (int32_t s = 0; s < graphs[i]->n; ++s) P.units.push_back(Unit{i, s, 1.0, -1});
         base[i + 1] = base[i] + graphs[i]->n;
     }
@@ -3301,7 +3310,7 @@ int fbc_sssp_debug(fbc_graph G, int32_t source, int32_t* out_dist, uint64_t* out
     P.seg_maxw.push_back(G->maxw);
     P.seg_maxindeg.push_back(G->maxindeg);
     P.seg_maxdeg.push_back(G->maxdeg);
-    P.seg_ties.push_back(G->ties);
+    P.seg_ties.push_back(0.0);
     P.units.push_back(Unit{0, source, 1.0, -1});
     P.bc_len = G->n;
     P.dbg_sig = (unsigned long long*)base;
